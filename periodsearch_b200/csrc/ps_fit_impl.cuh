@@ -43,6 +43,29 @@ __device__ __forceinline__ double rcp_newton(double x) {
 // the point-sort segment from the problem (DevProblem::fch, rt, sortseg):
 // runtime tile shapes, chosen by ps_autotune; no choice changes any result.
 
+// Quotients a / d of one divisor with IEEE rounding, as the reference's
+// divisions give them: y = RN(1 / d) (the hardware's approximate reciprocal, a
+// cubic and a final Newton step), then q = a y and one residual step
+// q + y (a - d q) in fused arithmetic, which rounds correctly when y does
+// (Markstein, IBM J. Res. Dev. 34, 1990).  For d in (2e-8, 4] and a of ordinary
+// magnitude (no overflow, underflow or special value anywhere on the way).
+// No branch and no call, unlike the division, so several run side by side.
+struct QuotientsBy {
+    double d, y;
+    __device__ __forceinline__ explicit QuotientsBy(double divisor) : d(divisor) {
+        double r;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+        double e = fma(-d, r, 1.0);
+        r = fma(r, fma(e, e, e), r);
+        e = fma(-d, r, 1.0);
+        y = fma(r, e, r);
+    }
+    __device__ __forceinline__ double of(double a) const {
+        const double q = a * y;
+        return fma(fma(-d, q, a), y, q);
+    }
+};
+
 // Blocks of the alpha/beta/chi2 accumulation for mfit free parameters: for
 // each even j0 <= mfit - 1, the 4-column blocks k0 = 4 kb of the lower
 // triangle (k0 <= j0 + 1) and the beta block k0 = kB; then the chi2 block
@@ -646,16 +669,27 @@ __device__ __forceinline__ void curv_phase(const DevProblem& P, const double* a,
 // sum), so both give the same bits; the fast form sums on one warp in a
 // fixed order.  The result lands in misc[M_CHISQ].
 template <bool kFast>
-__device__ __forceinline__ void chi2_rows(const DevProblem& P, const double* yt, double* misc) {
+__device__ __forceinline__ void chi2_rows(const DevProblem& P, const double* yt, double* misc, double* work) {
     if constexpr (!kFast) {
-        if (threadIdx.x == 0) {
-            double acc = 0;
-            for (int r = 0; r < P.n_rows; r++) {
-                const double dy = P.yobs[r] - yt[r];
-                acc = acc + dy * dy * P.sig2i[r] * P.wght[r];
+        // the terms by all threads, to shared memory; the sum by one (with its
+        // loads in global memory that thread took 75 cycles a row, 57 000 at 763
+        // rows and two fits per SM; the add chain itself is 8 a row)
+        constexpr int kBlock = 4 * kMf;
+        double acc = 0;
+        for (int r0 = 0; r0 < P.n_rows; r0 += kBlock) {
+            const int nr = min(kBlock, P.n_rows - r0);
+            __syncthreads();
+            for (int r = threadIdx.x; r < nr; r += kThreads) {
+                const double dy = P.yobs[r0 + r] - yt[r0 + r];
+                work[r] = dy * dy * P.sig2i[r0 + r] * P.wght[r0 + r];
             }
-            misc[M_CHISQ] = acc;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+#pragma unroll 8
+                for (int r = 0; r < nr; r++) acc = acc + work[r];
+            }
         }
+        if (threadIdx.x == 0) misc[M_CHISQ] = acc;
     } else {
         if (threadIdx.x < 32) {
             double acc = 0;
@@ -679,103 +713,145 @@ __device__ __forceinline__ void chi2_rows(const DevProblem& P, const double* yt,
 // 92-104) and chi2, with the operations and sum orders of evaluate(), so
 // that in the reference-order form every value is bit-identical to the one
 // evaluate() gives at the same point.  The model goes to yt; Jt is not
-// touched.  Thread per data point, facet normals staged in chunks of kMf.
+// touched.  Thread per data point, facet normals staged in chunks of kMf, four
+// facets at a time (model_facets).
 // Buffers (shared memory): g, area [F] (area is not padded past F here);
 // misc and B/D (blmatrix) as in evaluate(); work >= max(sortseg, 4 kMf,
 // kThreads) doubles, 16-byte aligned; perm sortseg ints.  Used by the FP64
 // fit kernels (evaluate_model) and the mixed-precision one.
+// Facets [0, kU) of `nrm` ({nx, ny, nz, Area}, zeros where there is no facet)
+// for one point per lane: the terms of all kU without a branch, so that their
+// chains run side by side, then the sum in facet order.  A facet that the lane
+// does not see adds Area 0 times a finite value, which leaves the sum as it is.
+// kPlain: see QuotientsBy.  Bound by the latency of one pair's chain: a warp that
+// took the facets one by one, with the IEEE division's branch, spent 470 cycles
+// on each at 118 points (one warp per scheduler), 135 000 of a step's 430 000.
+// Four at a time: one fit of 118 points and 288 facets 9.7 -> 7.6 ms, 600 fits
+// of 760 points and 800 facets 339 -> 314 ms.
+template <bool kFast, bool kPlain, int kU>
+__device__ __forceinline__ void model_facets(const double4* nrm, const double* e, const double* e0, double cl, double cls,
+                                             double& br) {
+    double mu[kU], mu0[kU], w[kU];
+    bool vis[kU], some = false;
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        const double4 n = nrm[u];
+        mu[u] = e[0] * n.x + e[1] * n.y + e[2] * n.z;
+        mu0[u] = e0[0] * n.x + e0[1] * n.y + e0[2] * n.z;
+        vis[u] = (mu[u] > kTinyD) && (mu0[u] > kTinyD);
+        w[u] = vis[u] ? n.w : 0.0;
+        some = some || vis[u];
+    }
+    if (!__any_sync(0xffffffffu, some)) return;
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        const double dnom = vis[u] ? mu[u] + mu0[u] : 1.0;
+        if constexpr (kFast) {
+            const double r = rcp_newton(dnom);
+            mu[u] = mu[u] * mu0[u] * fma(cls, r, cl);
+        } else {
+            const double s = mu[u] * mu0[u] * (cl + (kPlain ? QuotientsBy(dnom).of(cls) : cls / dnom));
+            mu[u] = w[u] * s;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        if constexpr (kFast)
+            br = fma(w[u], mu[u], br);
+        else
+            br = br + mu[u];
+    }
+}
+
+// The brightness of every data point to yt, with chck and the facet-area sum
+// on the way (four lanes of the last warp, facets in order).
+template <bool kFast, bool kPlain>
+__device__ __forceinline__ void model_points(const DevProblem& P, const double* area, double* misc, const double* B,
+                                             double* work, int* perm, double* yt) {
+    constexpr int kU = 4;  // facets at a time
+    const int tid = threadIdx.x, F = P.F, job = tid - (kThreads - 32);
+    const double cl = misc[M_CL], cls = misc[M_CLS];
+    double sum = 0;
+    // points in segments sorted by viewing direction (as in evaluate()), so
+    // that the points of a warp see nearly the same facets
+    for (int s0 = 0; s0 < P.n_points; s0 += P.sortseg) {
+        const int seg = min(P.sortseg, P.n_points - s0);
+        __syncthreads();
+        sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
+        // kMp points per thread at most (slot j of thread t: point base + j kThreads
+        // + t, so each slot's warp holds consecutive sorted points)
+        const int k = min(kMp, (seg + kThreads - 1) / kThreads);
+        for (int base = 0; base < seg; base += k * kThreads) {
+            double ej[kMp][3], fj[kMp][3], sc[kMp], br[kMp];
+#pragma unroll
+            for (int j = 0; j < kMp; j++) {
+                const int i = base + j * kThreads + tid;
+                br[j] = sc[j] = 0;
+#pragma unroll
+                for (int c = 0; c < 3; c++) ej[j][c] = fj[j][c] = 0;
+                if (j < k && i < seg) {
+                    PointGeom G;
+                    point_geometry(P, perm[i], B, B + 9, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        ej[j][c] = G.e[c];
+                        fj[j][c] = G.e0[c];
+                    }
+                    sc[j] = G.scale;
+                }
+            }
+            double4* nrm = reinterpret_cast<double4*>(work);  // [kMf] nx, ny, nz, Area
+            for (int c0 = 0; c0 < F; c0 += kMf) {
+                const int nf = min(kMf, F - c0);
+                __syncthreads();
+                for (int ff = tid; ff < ((nf + kU - 1) & ~(kU - 1)); ff += kThreads) {
+                    const double* fa = P.fac + (size_t)(c0 + ff) * 4;
+                    nrm[ff] = ff < nf ? make_double4(fa[0], fa[1], fa[2], area[c0 + ff]) : make_double4(0, 0, 0, 0);
+                }
+                __syncthreads();
+                if (s0 == 0 && base == 0 && job >= 0 && job < 4) {
+#pragma unroll 8
+                    for (int ff = 0; ff < nf; ff++) {
+                        const double* n = work + 4 * ff;
+                        if (job == 3)
+                            sum = sum + n[3];
+                        else if constexpr (kFast)
+                            sum = fma(n[3], n[job], sum);
+                        else
+                            sum = sum + n[3] * n[job];
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kMp; j++) {
+                    // a warp without points in this slot has nothing to do
+                    if (j >= k || base + j * kThreads + (tid & ~31) >= seg) continue;
+                    for (int ff = 0; ff < nf; ff += kU)
+                        model_facets<kFast, kPlain, kU>(nrm + ff, ej[j], fj[j], cl, cls, br[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kMp; j++) {
+                const int i = base + j * kThreads + tid;
+                if (j < k && i < seg) yt[perm[i]] = br[j] * sc[j];
+            }
+        }
+    }
+    if (job >= 0 && job < 4) misc[job < 3 ? M_CHK0 + job : M_SAREA] = sum;
+}
+
 template <bool kFast>
 __device__ void model_pass(const DevProblem& P, const double* a, double* g, double* area, double* misc, double* B,
                            double* D, double* work, int* perm, double* yt) {
     const int tid = threadIdx.x;
-    const int F = P.F, C = P.C;
-    eval_scalars(a, C, B, D, misc);
+    eval_scalars(a, P.C, B, D, misc);
     curv_phase(P, a, g, area, false);
     __syncthreads();
-    // chck and the facet-area sum, facets in order (as evaluate() and the
-    // fast point loop form them); four threads, loads ahead of the sums
-    if (tid < 4) {
-        double s = 0;
-        if (tid < 3) {
-#pragma unroll 8
-            for (int f = 0; f < F; f++) s = s + area[f] * __ldg(P.fac + (size_t)f * 4 + tid);
-            misc[M_CHK0 + tid] = s;
-        } else {
-#pragma unroll 8
-            for (int f = 0; f < F; f++) s = s + area[f];
-            misc[M_SAREA] = s;
-        }
-    }
-    const double cl = misc[M_CL], cls = misc[M_CLS];
-    // points in segments sorted by viewing direction (as in evaluate()), so
-    // that the points of a warp see nearly the same facets
-    for (int s0 = 0; s0 < P.n_points; s0 += P.sortseg) {
-    const int seg = min(P.sortseg, P.n_points - s0);
-    __syncthreads();
-    sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
-    // kMp points per thread at most (slot j of thread t: point base + j kThreads
-    // + t, so each slot's warp holds consecutive sorted points): independent
-    // chains per facet and one load of each facet for all of them
-    const int k = min(kMp, (seg + kThreads - 1) / kThreads);
-    for (int base = 0; base < seg; base += k * kThreads) {
-        int pj[kMp];
-        bool aj[kMp];
-        double ej[kMp][3], fj[kMp][3], sc[kMp], br[kMp];
-#pragma unroll
-        for (int j = 0; j < kMp; j++) {
-            const int i = base + j * kThreads + tid;
-            aj[j] = j < k && i < seg;
-            pj[j] = aj[j] ? perm[i] : 0;
-            br[j] = 0;
-            sc[j] = 0;
-#pragma unroll
-            for (int c = 0; c < 3; c++) ej[j][c] = fj[j][c] = 0;
-            if (aj[j]) {
-                PointGeom G;
-                point_geometry(P, pj[j], B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    ej[j][c] = G.e[c];
-                    fj[j][c] = G.e0[c];
-                }
-                sc[j] = G.scale;
-            }
-        }
-        double4* nrm = reinterpret_cast<double4*>(work);  // [kMf] nx, ny, nz, Area
-        for (int c0 = 0; c0 < F; c0 += kMf) {
-            const int nf = min(kMf, F - c0);
-            __syncthreads();
-            for (int ff = tid; ff < nf; ff += kThreads) {
-                const double* fa = P.fac + (size_t)(c0 + ff) * 4;
-                nrm[ff] = make_double4(fa[0], fa[1], fa[2], area[c0 + ff]);
-            }
-            __syncthreads();
-#pragma unroll 2
-            for (int ff = 0; ff < nf; ff++) {
-                const double4 n = nrm[ff];
-#pragma unroll
-                for (int j = 0; j < kMp; j++) {
-                    if (!aj[j]) continue;
-                    const double mu = ej[j][0] * n.x + ej[j][1] * n.y + ej[j][2] * n.z;
-                    const double mu0 = fj[j][0] * n.x + fj[j][1] * n.y + fj[j][2] * n.z;
-                    if ((mu > kTinyD) && (mu0 > kTinyD)) {
-                        if constexpr (kFast) {
-                            const double r = rcp_newton(mu + mu0);
-                            br[j] = fma(n.w, mu * mu0 * fma(cls, r, cl), br[j]);
-                        } else {
-                            const double dnom = mu + mu0;
-                            const double s = mu * mu0 * (cl + cls / dnom);
-                            br[j] = br[j] + n.w * s;
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kMp; j++)
-            if (aj[j]) yt[pj[j]] = br[j] * sc[j];
-    }
-    }
+    const double cls = misc[M_CLS];
+    if (kFast || (fabs(cls) > 1e-200 && fabs(cls) < 1e200))
+        model_points<kFast, true>(P, area, misc, B, work, perm, yt);
+    else
+        model_points<kFast, false>(P, area, misc, B, work, perm, yt);
     __syncthreads();
     if (tid < 3) yt[P.n_points + tid] = misc[M_CHK0 + tid];
     // relative-lightcurve normalisation of the model, mrqcof.c:53-58, 92-104
@@ -800,7 +876,7 @@ __device__ void model_pass(const DevProblem& P, const double* a, double* g, doub
         }
     }
     __syncthreads();
-    chi2_rows<kFast>(P, yt, misc);
+    chi2_rows<kFast>(P, yt, misc, work);
     __syncthreads();
 }
 
@@ -1063,7 +1139,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
         // chi2 as the model-only pass sums it, so that the LM test compares
         // values of one rounding
         __syncthreads();
-        chi2_rows<true>(P, yt, misc);
+        chi2_rows<true>(P, yt, misc, work);
     } else {
         // alpha = J^T W J, beta = J^T W dy, chi2 (mrqcof.c:106-147), every entry
         // summing the rows in order.  Tile of kRt rows: Ws[r][j] = (J[r][l_j]
