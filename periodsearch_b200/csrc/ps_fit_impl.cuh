@@ -894,28 +894,48 @@ __device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, i
                       (int*)(sm + L.perm), ym);
 }
 
-// bright.c:54-125 for every data point in the reference's operation order
-// (PS_FORM_FP64), in segments of points sorted by viewing direction.  Two
-// threads per point: thread t works on point slot t mod 128 of a pass of 128
-// points, and its half h = t / 128 (warps 0-3, warps 4-7) keeps the shape
-// sums of coefficients [h NCB/2, (h + 1) NCB/2) and half of the other
-// per-point sums (h = 0: the brightness and the rotation derivatives 0 and 1;
-// h = 1: rotation derivative 2 and the two scattering sums).  Every sum runs
-// over the facets in order with the reference's operations, each in one
-// thread, so the results are the bits of one thread per point; both halves
-// form the per-pair terms (visibility, s, the derivative factors).  Each half
-// runs its own instantiation of the pass (H), so that a thread holds only its
-// half's state and its accumulators fit in 128 registers (two fits per SM);
-// both execute the same block barriers, warp by warp.
-template <int NCB, int H>
-__device__ __forceinline__ void ref_pass(const DevProblem& P, const double* B, const double* D, double* misc,
-                                         const double* g, const double* area, double* s_fac, double* s_dg,
-                                         double* sdv, int pl, bool act, int p, double* Jt, double* yt) {
-    constexpr int KH = NCB / 2;
+// bright.c:54-125 in the reference's operation order (PS_FORM_FP64) for a pass
+// of 128 data points, two threads per point: thread t works on point slot
+// t mod 128, and its half H = t / 128 (warps 0-3, warps 4-7) keeps the shape
+// sums of kCount coefficients from kFirst and half of the other per-point
+// sums (H = 0: the brightness and the rotation derivatives 0 and 1; H = 1:
+// rotation derivative 2 and the scattering sums).  Every sum runs over the
+// facets in order with the reference's operations, each in one thread, so the
+// results are the bits of one thread per point; both halves form the per-pair
+// terms (visibility, s, the derivative factors), of kU facets at a time, with
+// one reciprocal per pair (QuotientsBy) and no branch, so that their chains run
+// side by side.  Out of line, an instantiation per half: a thread holds only
+// its half's state, which fits 128 registers (two fits per SM); inlined into
+// evaluate, spilled values were reloaded once per facet.  600 fits of 760
+// points, 800 facets and 49 coefficients: 314 ms with one facet at a time, three
+// or four IEEE divisions each, inlined; 277 with two facets and one reciprocal;
+// 261 out of line; 253 with the halves balanced (ref_halves; one facet: 286,
+// four: 276, which need more than 128 registers).  With few coefficients four
+// fit: 500 points and 16 coefficients, 140 fits and 400: 112 -> 109 ms.
+// `p`: the thread's point, -1 for none.  want_cl, all: also the columns of the
+// Lambert coefficient, of the (never fitted) Lommel-Seeliger one.
+template <int NCB, int H, int kFirst, int kCount>
+__device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool want_cl, bool all, double* Jt,
+                                      double* yt) {
+    extern __shared__ __align__(16) double sm[];
+    const DevProblem& P = *Pp;
+    const Layout L = make_layout(P);
+    const double* B = sm + L.blm;
+    const double* D = B + 9;
+    const double* misc = sm + L.misc;
+    const double* g = sm + L.g;
+    const double* area = sm + L.area;
+    double* s_fac = sm + L.work;
+    double* s_dg = s_fac + kFch * 5;
+    double* sdv = s_fac + ((kFch * 5 + kFch * NCB + 1) & ~1);
+    const int pl = threadIdx.x & (kThreads / 2 - 1);
+    const bool act = p >= 0;
     constexpr int kPts = kThreads / 2;
+    constexpr int kU = NCB <= 24 ? 4 : 2;  // facets at a time
     const int tid = threadIdx.x;
     const int F = P.F, C = P.C, npad = P.npad;
     const double cl = misc[M_CL], cls = misc[M_CLS];
+    const bool finite = isfinite(cls);  // cls / d is cls where it is not
     constexpr int c0 = H == 0 ? 0 : 2;  // the rotation derivative both halves keep
     // this point's derivative vectors in shared memory ([vector][slot]: the
     // loads of a warp are consecutive): H = 0 columns 0 and 1 of de, de0
@@ -937,9 +957,9 @@ __device__ __forceinline__ void ref_pass(const DevProblem& P, const double* B, c
             }
         }
     }
-    double acc[KH];
+    double acc[kCount > 0 ? kCount : 1];
 #pragma unroll
-    for (int k = 0; k < KH; k++) acc[k] = 0;
+    for (int k = 0; k < kCount; k++) acc[k] = 0;
     double a0 = 0, a1 = 0, a2 = 0;  // H = 0: br, rot0, rot1; H = 1: s_cl, rot2, s_cls
     for (int f0 = 0; f0 < F; f0 += kFch) {
         const int nf = min(kFch, F - f0);
@@ -957,37 +977,56 @@ __device__ __forceinline__ void ref_pass(const DevProblem& P, const double* B, c
             s_fac[ff * 5 + 4] = fa[3];
         }
         __syncthreads();
-        if (act) {
-#pragma unroll 2  // two facets in flight (1.9 % on c2; same operations per sum)
-            for (int ff = 0; ff < nf; ff++) {
-                const double nx = s_fac[ff * 5 + 0], ny = s_fac[ff * 5 + 1], nz = s_fac[ff * 5 + 2];
-                const double mu = e[0] * nx + e[1] * ny + e[2] * nz;
-                const double mu0 = e0[0] * nx + e0[1] * ny + e0[2] * nz;
-                if ((mu > kTinyD) && (mu0 > kTinyD)) {
-                    const double ar = s_fac[ff * 5 + 3], darea = s_fac[ff * 5 + 4];
-                    const double dnom = mu + mu0;
-                    const double s = mu * mu0 * (cl + cls / dnom);
-                    const double q0 = mu0 / dnom, q1 = mu / dnom;
-                    const double dsmu = cls * (q0 * q0) + cl * mu0;
-                    const double dsmu0 = cls * (q1 * q1) + cl * mu;
-                    const double dbr = darea * s;
-                    const double* dg = s_dg + ff * NCB + H * KH;
+        // kU facets at a time: their per-pair terms without a branch, side by side,
+        // then the sums, facet by facet
+        for (int f1 = 0; f1 < nf; f1 += kU) {
+            const double* fq = s_fac + f1 * 5;
+            double sv[kU], dsmu[kU], dsmu0[kU];
+            bool vis[kU], some = false;
 #pragma unroll
-                    for (int k = 0; k < KH; k++) acc[k] = acc[k] + dbr * dg[k];
-                    {
-                        const double sum = nx * dv[0] + ny * dv[kPts] + nz * dv[2 * kPts];
-                        const double sum0 = nx * dv[3 * kPts] + ny * dv[4 * kPts] + nz * dv[5 * kPts];
-                        a1 = a1 + ar * (dsmu * sum + dsmu0 * sum0);
-                    }
-                    if constexpr (H == 0) {
-                        a0 = a0 + ar * s;
-                        const double sum = nx * dv[6 * kPts] + ny * dv[7 * kPts] + nz * dv[8 * kPts];
-                        const double sum0 = nx * dv[9 * kPts] + ny * dv[10 * kPts] + nz * dv[11 * kPts];
-                        a2 = a2 + ar * (dsmu * sum + dsmu0 * sum0);
-                    } else {
-                        a0 = a0 + mu * mu0 * ar;
-                        a2 = a2 + ar * mu * mu0 / (mu + mu0);
-                    }
+            for (int u = 0; u < kU; u++) {
+                const double* fp = fq + 5 * u;
+                sv[u] = e[0] * fp[0] + e[1] * fp[1] + e[2] * fp[2];     // mu
+                dsmu[u] = e0[0] * fp[0] + e0[1] * fp[1] + e0[2] * fp[2];  // mu0
+                vis[u] = (u == 0 || f1 + u < nf) && (sv[u] > kTinyD) && (dsmu[u] > kTinyD);
+                some = some || vis[u];
+            }
+            if (!__any_sync(0xffffffffu, some)) continue;
+            double cmu[kU], cmu0[kU];  // for the scattering sums (H = 1)
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const double mu = sv[u], mu0 = dsmu[u];
+                const double dnom = vis[u] ? mu + mu0 : 1.0;
+                const QuotientsBy by(dnom);
+                const double q0 = by.of(mu0), q1 = by.of(mu);
+                sv[u] = mu * mu0 * (cl + (finite ? by.of(cls) : cls * by.y));
+                dsmu[u] = cls * (q0 * q0) + cl * mu0;
+                dsmu0[u] = cls * (q1 * q1) + cl * mu;
+                cmu[u] = mu;
+                cmu0[u] = mu0;
+            }
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                if (!vis[u]) continue;
+                const double* fp = fq + 5 * u;
+                const double nx = fp[0], ny = fp[1], nz = fp[2], ar = fp[3], darea = fp[4];
+                const double dbr = darea * sv[u];
+                const double* dg = s_dg + (f1 + u) * NCB + kFirst;
+#pragma unroll
+                for (int k = 0; k < kCount; k++) acc[k] = acc[k] + dbr * dg[k];
+                {
+                    const double sum = nx * dv[0] + ny * dv[kPts] + nz * dv[2 * kPts];
+                    const double sum0 = nx * dv[3 * kPts] + ny * dv[4 * kPts] + nz * dv[5 * kPts];
+                    a1 = a1 + ar * (dsmu[u] * sum + dsmu0[u] * sum0);
+                }
+                if constexpr (H == 0) {
+                    a0 = a0 + ar * sv[u];
+                    const double sum = nx * dv[6 * kPts] + ny * dv[7 * kPts] + nz * dv[8 * kPts];
+                    const double sum0 = nx * dv[9 * kPts] + ny * dv[10 * kPts] + nz * dv[11 * kPts];
+                    a2 = a2 + ar * (dsmu[u] * sum + dsmu0[u] * sum0);
+                } else {
+                    if (want_cl) a0 = a0 + cmu[u] * cmu0[u] * ar;
+                    if (all) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
                 }
             }
         }
@@ -997,8 +1036,8 @@ __device__ __forceinline__ void ref_pass(const DevProblem& P, const double* B, c
         point_geometry(P, p, B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
         const double sc = G.scale;
 #pragma unroll
-        for (int k = 0; k < KH; k++)
-            if (H * KH + k < C) Jt[(size_t)(H * KH + k) * npad + p] = sc * acc[k];
+        for (int k = 0; k < kCount; k++)
+            if (kFirst + k < C) Jt[(size_t)(kFirst + k) * npad + p] = sc * acc[k];
         if constexpr (H == 0) {
             Jt[(size_t)(C + 0) * npad + p] = sc * a1;
             Jt[(size_t)(C + 1) * npad + p] = sc * a2;
@@ -1014,34 +1053,145 @@ __device__ __forceinline__ void ref_pass(const DevProblem& P, const double* B, c
     }
 }
 
+// Both halves of a pass over kTotal coefficients.  Half 0's extra rotation
+// derivative and brightness sum are 17 operations per pair, the shape sums 2
+// each, so half 1 takes eight more of them.
+template <int NCB, int kTotal>
+__device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool want_cl, bool all,
+                                           double* Jt, double* yt) {
+    constexpr int k0 = kTotal > 9 ? (kTotal - 8) / 2 & ~1 : 0;  // even: dg is read in pairs
+    if (h == 0)
+        ref_pass<NCB, 0, 0, k0>(Pp, p, want_cl, all, Jt, yt);
+    else
+        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, want_cl, all, Jt, yt);
+}
+
+// ref_pass over every data point, in segments sorted by viewing direction.
 template <int NCB>
-__device__ __forceinline__ void point_loop_ref(const DevProblem& P, double* sm, const Layout& L, const double* B,
-                                               const double* D, double* misc, const double* g, const double* area,
-                                               double* work, double* Jt, double* yt) {
+__device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp, double* sm, const Layout& L, bool all,
+                                               double* Jt, double* yt) {
     constexpr int kPts = kThreads / 2;
+    const DevProblem& P = *Pp;
     const int tid = threadIdx.x, h = tid / kPts, pl = tid - h * kPts;
-    double* s_fac = work;
-    double* s_dg = work + kFch * 5;
-    double* sdv = work + ((kFch * 5 + kFch * NCB + 1) & ~1);
+    const double* B = sm + L.blm;
+    const double* misc = sm + L.misc;
+    double* work = sm + L.work;
     int* perm = (int*)(sm + L.perm);
+    const bool want_cl = all || P.free_idx[P.mfit - 1] >= P.C + 6;
     for (int s0 = 0; s0 < P.n_points; s0 += P.sortseg) {
         const int seg = min(P.sortseg, P.n_points - s0);
         __syncthreads();
         sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
         for (int base = 0; base < seg; base += kPts) {
-            const bool act = base + pl < seg;
-            const int p = act ? perm[base + pl] : 0;
-            if (h == 0)
-                ref_pass<NCB, 0>(P, B, D, misc, g, area, s_fac, s_dg, sdv, pl, act, p, Jt, yt);
+            const int p = base + pl < seg ? perm[base + pl] : -1;
+            // C = 1 mod 8 for every even lmax = mmax: no sums for the padding
+            if (P.C > NCB - 7)
+                ref_halves<NCB, NCB>(Pp, h, p, want_cl, all, Jt, yt);
             else
-                ref_pass<NCB, 1>(P, B, D, misc, g, area, s_fac, s_dg, sdv, pl, act, p, Jt, yt);
+                ref_halves<NCB, NCB - 7>(Pp, h, p, want_cl, all, Jt, yt);
+        }
+    }
+}
+
+// alpha, beta and chi2 of the reference-order form from J^T and y; out of line
+// for its accumulators' registers.
+template <int NCB>
+__device__ __noinline__ void ref_alpha(const DevProblem* __restrict__ Pp, int alpha_off, int beta_off, const double* Jt,
+                                       const double* yt) {
+    extern __shared__ __align__(16) double sm[];
+    const DevProblem& P = *Pp;
+    const Layout L = make_layout(P);
+    const int tid = threadIdx.x, mfit = P.mfit, npad = P.npad;
+    double* alpha_out = sm + alpha_off;
+    double* beta_out = sm + beta_off;
+    double* misc = sm + L.misc;
+    double* work = sm + L.work;
+    // alpha = J^T W J, beta = J^T W dy, chi2 (mrqcof.c:106-147), every entry
+    // summing the rows in order.  Tile of kRt rows: Ws[r][j] = (J[r][l_j]
+    // sig2i) wght (j < mfit), Ws[r][jC] = dy dy sig2i wght; Js[r][k] =
+    // J[r][l_k] (k < mfit), Js[r][kB] = dy, Js[r][kB+1] = 1; other columns 0.
+    // Each job is a 2 x 4 block of entries (Ws columns j0, j0+1 against Js
+    // columns k0..k0+3), held in registers across the tiles.
+    const int kB = (mfit + 1) & ~1, jC = kB;
+    const int wst = jC + 2, jst = kB + 4;
+    double* Ws = work;
+    double* Js = work + kRt * wst;
+    const int* jobs = (const int*)(sm + L.ent);
+    const int njob = alpha_job_count(mfit);
+    constexpr int kJobs = kJobsFor<NCB>;
+    double acc2[kJobs][2][4];
+#pragma unroll
+    for (int q = 0; q < kJobs; q++)
+#pragma unroll
+        for (int a2 = 0; a2 < 2; a2++)
+#pragma unroll
+            for (int b4 = 0; b4 < 4; b4++) acc2[q][a2][b4] = 0;
+    for (int r0 = 0; r0 < P.n_rows; r0 += kRt) {
+        const int nr = min(kRt, P.n_rows - r0);
+        __syncthreads();
+        for (int idx = tid; idx < nr * mfit; idx += kThreads) {
+            const int j = idx / nr, r = idx - j * nr;
+            const int row = r0 + r;
+            const double d = Jt[(size_t)P.free_idx[j] * npad + row];
+            Js[r * jst + j] = d;
+            Ws[r * wst + j] = d * P.sig2i[row] * P.wght[row];
+        }
+        for (int r = tid; r < nr; r += kThreads) {
+            const int row = r0 + r;
+            const double dy = P.yobs[row] - yt[row];
+            for (int k = mfit; k < jst; k++) Js[r * jst + k] = k == kB ? dy : (k == kB + 1 ? 1.0 : 0.0);
+            for (int j = mfit; j < wst; j++) Ws[r * wst + j] = j == jC ? dy * dy * P.sig2i[row] * P.wght[row] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kJobs; q++) {
+            const int e = tid + q * kThreads;
+            if (e < njob) {
+                const int j0 = jobs[e] & 0xffff, k0 = jobs[e] >> 16;
+                const double* wp = Ws + j0;
+                const double* jp = Js + k0;
+                for (int r = 0; r < nr; r++) {
+                    const double2 w = *reinterpret_cast<const double2*>(wp + r * wst);
+                    const double2 ja = *reinterpret_cast<const double2*>(jp + r * jst);
+                    const double2 jb = *reinterpret_cast<const double2*>(jp + r * jst + 2);
+                    const double wv[2] = {w.x, w.y}, jv[4] = {ja.x, ja.y, jb.x, jb.y};
+#pragma unroll
+                    for (int a2 = 0; a2 < 2; a2++)
+#pragma unroll
+                        for (int b4 = 0; b4 < 4; b4++) acc2[q][a2][b4] = acc2[q][a2][b4] + wv[a2] * jv[b4];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kJobs; q++) {
+        const int e = tid + q * kThreads;
+        if (e < njob) {
+            const int j0 = jobs[e] & 0xffff, k0 = jobs[e] >> 16;
+#pragma unroll
+            for (int a2 = 0; a2 < 2; a2++)
+#pragma unroll
+                for (int b4 = 0; b4 < 4; b4++) {
+                    const int j = j0 + a2, k = k0 + b4;
+                    const double v = acc2[q][a2][b4];
+                    if (j < mfit && k < mfit) {
+                        if (k <= j) {
+                            alpha_out[j * mfit + k] = v;
+                            alpha_out[k * mfit + j] = v;
+                        }
+                    } else if (j < mfit && k == kB) {
+                        beta_out[j] = v;
+                    } else if (j == jC && k == kB + 1) {
+                        misc[M_CHISQ] = v;
+                    }
+                }
         }
     }
 }
 
 template <int NCB, bool kFast>
 __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_off, int alpha_off, int beta_off,
-                                      double* Jt, double* yt) {
+                                      bool all, double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const double* a = sm + a_off;
     double* alpha_out = sm + alpha_off;
@@ -1096,7 +1246,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
             point_loop_fast<NCB, false>(P, sm, L, B, D, misc, g, area, dres, work, Jt, yt);
         }
     } else {
-        point_loop_ref<NCB>(P, sm, L, B, D, misc, g, area, work, Jt, yt);
+        point_loop_ref<NCB>(Pp, sm, L, all, Jt, yt);
     }
     __syncthreads();
     // convexity rows (conv.c:12-29): y = residual, J = dres for the shape
@@ -1141,87 +1291,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
         __syncthreads();
         chi2_rows<true>(P, yt, misc, work);
     } else {
-        // alpha = J^T W J, beta = J^T W dy, chi2 (mrqcof.c:106-147), every entry
-        // summing the rows in order.  Tile of kRt rows: Ws[r][j] = (J[r][l_j]
-        // sig2i) wght (j < mfit), Ws[r][jC] = dy dy sig2i wght; Js[r][k] =
-        // J[r][l_k] (k < mfit), Js[r][kB] = dy, Js[r][kB+1] = 1; other columns 0.
-        // Each job is a 2 x 4 block of entries (Ws columns j0, j0+1 against Js
-        // columns k0..k0+3), held in registers across the tiles.
-        const int kB = (mfit + 1) & ~1, jC = kB;
-        const int wst = jC + 2, jst = kB + 4;
-        double* Ws = work;
-        double* Js = work + kRt * wst;
-        const int* jobs = (const int*)(sm + L.ent);
-        const int njob = alpha_job_count(mfit);
-        constexpr int kJobs = kJobsFor<NCB>;
-        double acc2[kJobs][2][4];
-    #pragma unroll
-        for (int q = 0; q < kJobs; q++)
-    #pragma unroll
-            for (int a2 = 0; a2 < 2; a2++)
-    #pragma unroll
-                for (int b4 = 0; b4 < 4; b4++) acc2[q][a2][b4] = 0;
-        for (int r0 = 0; r0 < P.n_rows; r0 += kRt) {
-            const int nr = min(kRt, P.n_rows - r0);
-            __syncthreads();
-            for (int idx = tid; idx < nr * mfit; idx += kThreads) {
-                const int j = idx / nr, r = idx - j * nr;
-                const int row = r0 + r;
-                const double d = Jt[(size_t)P.free_idx[j] * npad + row];
-                Js[r * jst + j] = d;
-                Ws[r * wst + j] = d * P.sig2i[row] * P.wght[row];
-            }
-            for (int r = tid; r < nr; r += kThreads) {
-                const int row = r0 + r;
-                const double dy = P.yobs[row] - yt[row];
-                for (int k = mfit; k < jst; k++) Js[r * jst + k] = k == kB ? dy : (k == kB + 1 ? 1.0 : 0.0);
-                for (int j = mfit; j < wst; j++) Ws[r * wst + j] = j == jC ? dy * dy * P.sig2i[row] * P.wght[row] : 0.0;
-            }
-            __syncthreads();
-    #pragma unroll
-            for (int q = 0; q < kJobs; q++) {
-                const int e = tid + q * kThreads;
-                if (e < njob) {
-                    const int j0 = jobs[e] & 0xffff, k0 = jobs[e] >> 16;
-                    const double* wp = Ws + j0;
-                    const double* jp = Js + k0;
-                    for (int r = 0; r < nr; r++) {
-                        const double2 w = *reinterpret_cast<const double2*>(wp + r * wst);
-                        const double2 ja = *reinterpret_cast<const double2*>(jp + r * jst);
-                        const double2 jb = *reinterpret_cast<const double2*>(jp + r * jst + 2);
-                        const double wv[2] = {w.x, w.y}, jv[4] = {ja.x, ja.y, jb.x, jb.y};
-    #pragma unroll
-                        for (int a2 = 0; a2 < 2; a2++)
-    #pragma unroll
-                            for (int b4 = 0; b4 < 4; b4++) acc2[q][a2][b4] = acc2[q][a2][b4] + wv[a2] * jv[b4];
-                    }
-                }
-            }
-        }
-    #pragma unroll
-        for (int q = 0; q < kJobs; q++) {
-            const int e = tid + q * kThreads;
-            if (e < njob) {
-                const int j0 = jobs[e] & 0xffff, k0 = jobs[e] >> 16;
-    #pragma unroll
-                for (int a2 = 0; a2 < 2; a2++)
-    #pragma unroll
-                    for (int b4 = 0; b4 < 4; b4++) {
-                        const int j = j0 + a2, k = k0 + b4;
-                        const double v = acc2[q][a2][b4];
-                        if (j < mfit && k < mfit) {
-                            if (k <= j) {
-                                alpha_out[j * mfit + k] = v;
-                                alpha_out[k * mfit + j] = v;
-                            }
-                        } else if (j < mfit && k == kB) {
-                            beta_out[j] = v;
-                        } else if (j == jC && k == kB + 1) {
-                            misc[M_CHISQ] = v;
-                        }
-                    }
-            }
-        }
+        ref_alpha<NCB>(Pp, alpha_off, beta_off, Jt, yt);
     }
     __syncthreads();
 }
@@ -1345,7 +1415,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
         while (((niter < P.n_iter_max) && (iter_diff > P.iter_diff_max)) || (niter < P.n_iter_min)) {
             if (alamda < 0) {
                 alamda = P.alamda_start;
-                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), Jt, yt);
+                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), false, Jt, yt);
                 ochisq = misc[M_CHISQ];
                 cur0 = misc[M_CHK0];
                 cur1 = misc[M_CHK0 + 1];
@@ -1355,7 +1425,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
             } else if (j_stale) {
                 // alpha and beta at the point accepted last (its chi2, chck and
                 // area sum came from the model-only evaluation and are kept)
-                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), Jt, yt);
+                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), false, Jt, yt);
                 j_stale = false;
             }
             for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
@@ -1451,7 +1521,7 @@ __global__ void __launch_bounds__(kThreads, 1) eval_kernel(const DevProblem* __r
     alpha_jobs(P.mfit, (int*)(sm + L.ent));
     for (int i = tid; i < P.ma; i += kThreads) cg[i] = E.a[i];
     __syncthreads();
-    evaluate<NCB, kFast>(Pp, L.cg, L.alpha, L.beta, Jt, yt);
+    evaluate<NCB, kFast>(Pp, L.cg, L.alpha, L.beta, true, Jt, yt);
     for (int i = tid; i < P.mfit * P.mfit; i += kThreads) E.alpha[i] = sm[L.alpha + i];
     for (int i = tid; i < P.mfit; i += kThreads) E.beta[i] = sm[L.beta + i];
     if (tid == 0) E.chisq[0] = sm[L.misc + M_CHISQ];

@@ -33,3 +33,31 @@ def test_short_fits_follow_the_oracle(native, oracle_lib, tmp_path, form, nrows,
         if ro["status"] == 0:
             assert np.linalg.norm(cg - cg_o) <= 1e-6 * np.linalg.norm(cg_o)
     g.close()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fast"])
+@pytest.mark.parametrize("nrows,lmax,points", [(2, 1, 127), (3, 2, 129), (5, 4, 130), (6, 6, 66)])
+def test_jacobian_rows_at_any_scattering(native, oracle_lib, tmp_path, form, nrows, lmax, points):
+    """Every row and column of J, with scattering coefficients that a fit does
+    not take: the reference-order form's quotients must round like divisions
+    there too.  Points around the 128 of a pass; coefficient counts with and
+    without padding (4, 9, 25, 49 of 8, 16, 32, 56)."""
+    w = synth.make_workload("jac", 60 + lmax, dense_lcs=1, dense_pts=20, sparse_pts=points - 20, years=6, true_lmax=2,
+                            fit_lmax=lmax, nrows=nrows, noise=0.02, n_periods=2)
+    path = synth.write_input(w, str(tmp_path))
+    o = oracle_lib.Oracle(path)
+    o.set_conw_r(o.conw_r)
+    g = native.PeriodSearch(path, form={"fp64": native.PS_FORM_FP64, "fast": native.PS_FORM_FAST}[form])
+    g.set_conw_r(o.conw_r)
+    a = o.initial_parameters(o.freq(1), 6)
+    C = g.ncoef
+    for log_cl, cls in ((np.log(0.1), 1.0), (-3.0, 0.0), (0.7, 3.7e5), (-1.0, 1e-12)):
+        a[C + 6], a[C + 7] = log_cl, cls
+        y_o, J_o = o.model(a)
+        y, J = g.model(a)
+        assert np.linalg.norm(y - y_o) <= 1e-11 * np.linalg.norm(y_o)
+        for k in range(g.ma):
+            # a column may be what cancellation leaves: its scale is J's at least
+            scale = max(np.linalg.norm(J_o[:, k]), 1e-3 * np.linalg.norm(J_o) / np.sqrt(g.ma))
+            assert np.linalg.norm(J[:, k] - J_o[:, k]) <= 1e-11 * scale, (log_cl, cls, k)
+    g.close()
