@@ -282,12 +282,16 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // FP64 tensor cores.  The shape derivatives are a matrix product,
 //   dyda[p][k] = sum_f (Darea_f s_pf) (g_f dsph[f][k]) = sum_f A[p][f] dsph[f][k]
 // with A[p][f] = Area_f s_pf for the facets p sees (0 otherwise).  A warp owns
-// kMT tiles of 8 points; per step of 4 facets lane (g, q) forms A for point g
-// and facet q of each tile -- visibility, s, and the brightness, rotation and
-// scattering sums over its facets -- and the warp multiplies the 8x4 A tile
-// into the 8 x NCB accumulator tiles with m8n8k4 FP64 MMAs (B = dsph rows from
-// shared memory).  A tile with no visible (point, facet) pair in the step
-// skips its MMAs.  Facet chunks are staged with asynchronous copies, one chunk
+// 8 points; per step of 4 facets lane (g, q) forms A for point g and facet q
+// -- visibility, s, and the brightness, rotation and scattering sums over its
+// facets -- and the warp multiplies the 8x4 A tile into the 8 x NCB accumulator
+// tiles with m8n8k4 FP64 MMAs (B = dsph rows from shared memory).  A step with
+// no visible (point, facet) pair skips its MMAs.  Out of line, for the
+// registers.  Bound by the latency of a step's chain and by instruction issue;
+// one reciprocal without a branch instead of the IEEE division's: 140 fits of
+// 20 000 points, 2048 facets and 81 coefficients 304 -> 258 ms, 2400 fits of 760
+// points, 800 facets and 49 coefficients unchanged (92 ms; there two steps go
+// side by side, which one CTA per SM does not need: 262 ms).  Facet chunks are staged with asynchronous copies, one chunk
 // ahead.  Sums split by facet (lane q takes facets q mod 4) are combined at
 // the end: the form differs from the reference order by rounding only.
 // kX1 (C = NCB - 7, i.e. C = 1 mod 8 as for every even lmax = mmax): the last
@@ -295,14 +299,21 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // summed per lane on the FP64 pipe (one FMA per visible pair) and the MMA
 // sequence covers the first NCB - 8 columns.
 template <int NCB, bool kX1>
-__device__ __forceinline__ void point_loop_fast(const DevProblem& P, double* sm, const Layout& L, const double* B,
-                                                const double* D, double* misc, const double* g_f,
-                                                const double* area, double* dres, double* work, double* Jt,
-                                                double* yt) {
+__device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, double* Jt, double* yt) {
+    extern __shared__ __align__(16) double sm[];
+    const DevProblem& P = *Pp;
+    const Layout L = make_layout(P);
+    double* misc = sm + L.misc;
+    const double* B = sm + L.blm;
+    const double* D = B + 9;
+    const double* g_f = sm + L.g;
+    const double* area = sm + L.area;
+    double* dres = sm + L.dres;
+    double* work = sm + L.work;
     constexpr int NT = kX1 ? NCB / 8 - 1 : NCB / 8;  // MMA accumulator tiles per 8 points
     static_assert(NT > 0, "kX1 needs NCB >= 16");
-    constexpr int kMT = 1;                       // point tiles per warp
-    constexpr int kPts = (kThreads / 32) * 8 * kMT;  // points per pass
+    constexpr int kU = NCB <= 64 ? 2 : 1;            // steps of four facets at a time
+    constexpr int kPts = (kThreads / 32) * 8;        // points per pass
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, q = lane & 3;
     const int F = P.F, C = P.C, npad = P.npad;
@@ -325,36 +336,23 @@ __device__ __forceinline__ void point_loop_fast(const DevProblem& P, double* sm,
         __syncthreads();
         sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
         for (int base = 0; base < seg; base += kPts) {
-            int p[kMT];
-            bool act[kMT];
-            double e[kMT][3], e0[kMT][3];
+            const int ps = base + warp * 8 + g;
+            const bool act = ps < seg;
+            const int p = act ? perm[ps] : 0;
+            double e[3] = {0, 0, 0}, e0[3] = {0, 0, 0};
+            if (act) {
+                PointGeom G;
+                point_geometry(P, p, B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
 #pragma unroll
-            for (int i = 0; i < kMT; i++) {
-                const int ps = base + warp * 8 * kMT + i * 8 + g;
-                act[i] = ps < seg;
-                p[i] = act[i] ? perm[ps] : 0;
-#pragma unroll
-                for (int c = 0; c < 3; c++) e[i][c] = e0[i][c] = 0;
-                if (act[i]) {
-                    PointGeom G;
-                    point_geometry(P, p[i], B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        e[i][c] = G.e[c];
-                        e0[i][c] = G.e0[c];
-                    }
+                for (int c = 0; c < 3; c++) {
+                    e[c] = G.e[c];
+                    e0[c] = G.e0[c];
                 }
             }
-            double acc[kMT][NT][2];
-            double br[kMT], T[kMT][3], S[kMT][3], s_cl[kMT], s_cls[kMT], x1[kMT];
+            double acc[NT][2];
+            double br = 0, T[3] = {0, 0, 0}, S[3] = {0, 0, 0}, s_cl = 0, s_cls = 0, x1 = 0;
 #pragma unroll
-            for (int i = 0; i < kMT; i++) {
-#pragma unroll
-                for (int t = 0; t < NT; t++) acc[i][t][0] = acc[i][t][1] = 0;
-                br[i] = s_cl[i] = s_cls[i] = x1[i] = 0;
-#pragma unroll
-                for (int c = 0; c < 3; c++) T[i][c] = S[i][c] = 0;
-            }
+            for (int t = 0; t < NT; t++) acc[t][0] = acc[t][1] = 0;
             __syncthreads();
             stage_chunk_async<NCB>(P, 0, work, work + fch * 4);
             cp_async_wait_all();
@@ -389,97 +387,100 @@ __device__ __forceinline__ void point_loop_fast(const DevProblem& P, double* sm,
                 }
                 // Facets past F (zero rows in the staged chunk, zero area) and
                 // inactive lanes (e = e0 = 0) have mu = mu0 = 0: not visible.
-                for (int j = 0; j < nf; j += 4) {
-                    const int ff = j + q;
-                    const double nx = fb[ff * 4 + 0], ny = fb[ff * 4 + 1], nz = fb[ff * 4 + 2];
-                    const double ar = area[f0 + ff];
-                    double av[kMT];
-                    bool any[kMT];
+                // kU steps of four facets at a time: their per-pair terms without a
+                // branch, side by side (a facet the lane does not see counts with
+                // area 0, which leaves every sum as it is), then the MMAs.
+                for (int j = 0; j < nf; j += 4 * kU) {
+                    double mu[kU], mu0[kU], ar[kU], av[kU];
+                    bool any[kU], some = false;
 #pragma unroll
-                    for (int i = 0; i < kMT; i++) {
-                        const double mu = e[i][0] * nx + e[i][1] * ny + e[i][2] * nz;
-                        const double mu0 = e0[i][0] * nx + e0[i][1] * ny + e0[i][2] * nz;
-                        const bool vis = (mu > kTinyD) && (mu0 > kTinyD);
-                        any[i] = __any_sync(full, vis);
-                        av[i] = 0;
-                        if (vis) {
-                            const double r = 1.0 / (mu + mu0);
-                            const double sv = mu * mu0 * fma(cls, r, cl);
-                            av[i] = ar * sv;
-                            br[i] += av[i];
-                            const double q0 = mu0 * r, q1 = mu * r;
-                            const double w = ar * fma(cls * q0, q0, cl * mu0);
-                            const double w0 = ar * fma(cls * q1, q1, cl * mu);
-                            T[i][0] = fma(w, nx, T[i][0]);
-                            T[i][1] = fma(w, ny, T[i][1]);
-                            T[i][2] = fma(w, nz, T[i][2]);
-                            S[i][0] = fma(w0, nx, S[i][0]);
-                            S[i][1] = fma(w0, ny, S[i][1]);
-                            S[i][2] = fma(w0, nz, S[i][2]);
-                            const double mm = mu * mu0 * ar;
-                            s_cl[i] += mm;
-                            s_cls[i] = fma(mm, r, s_cls[i]);
-                            if (kX1) x1[i] = fma(av[i], db[ff * kDs<NCB> + 8 * NT], x1[i]);
-                        }
+                    for (int u = 0; u < kU; u++) {
+                        const int ff = j + 4 * u + q;
+                        const bool in = kU == 1 || j + 4 * u < nf;
+                        const double* n = fb + (in ? ff : q) * 4;
+                        mu[u] = fma(e[2], n[2], fma(e[0], n[0], e[1] * n[1]));
+                        mu0[u] = fma(e0[2], n[2], fma(e0[0], n[0], e0[1] * n[1]));
+                        const bool vis = in && (mu[u] > kTinyD) && (mu0[u] > kTinyD);
+                        any[u] = __any_sync(full, vis);
+                        some = some || any[u];
+                        ar[u] = vis ? area[f0 + ff] : 0.0;
+                        av[u] = vis ? mu[u] + mu0[u] : 1.0;
                     }
-                    bool some = false;
-#pragma unroll
-                    for (int i = 0; i < kMT; i++) some = some || any[i];
                     if (!some) continue;
-                    const double* brow = db + ff * kDs<NCB> + g;
 #pragma unroll
-                    for (int t = 0; t < NT; t++) {
-                        const double bv = brow[t * 8];
+                    for (int u = 0; u < kU; u++) av[u] = QuotientsBy(av[u]).y;
 #pragma unroll
-                        for (int i = 0; i < kMT; i++)
-                            if (any[i]) dmma_8x8x4(acc[i][t][0], acc[i][t][1], av[i], bv);
+                    for (int u = 0; u < kU; u++) {
+                        const int ff = j + 4 * u + q;
+                        const double* n = fb + (kU == 1 || j + 4 * u < nf ? ff : q) * 4;
+                        const double r = av[u];
+                        const double sv = mu[u] * mu0[u] * fma(cls, r, cl);
+                        av[u] = ar[u] * sv;
+                        br = __dadd_rn(br, av[u]);
+                        const double q0 = mu0[u] * r, q1 = mu[u] * r;
+                        const double w = ar[u] * fma(cls * q0, q0, cl * mu0[u]);
+                        const double w0 = ar[u] * fma(cls * q1, q1, cl * mu[u]);
+                        T[0] = fma(w, n[0], T[0]);
+                        T[1] = fma(w, n[1], T[1]);
+                        T[2] = fma(w, n[2], T[2]);
+                        S[0] = fma(w0, n[0], S[0]);
+                        S[1] = fma(w0, n[1], S[1]);
+                        S[2] = fma(w0, n[2], S[2]);
+                        const double mm = mu[u] * mu0[u] * ar[u];
+                        s_cl += mm;
+                        s_cls = fma(mm, r, s_cls);
+                        if (kX1) x1 = fma(av[u], db[(kU == 1 || j + 4 * u < nf ? ff : q) * kDs<NCB> + 8 * NT], x1);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kU; u++) {
+                        if (!any[u]) continue;
+                        const double* brow = db + (j + 4 * u + q) * kDs<NCB> + g;
+#pragma unroll
+                        for (int t = 0; t < NT; t++) dmma_8x8x4(acc[t][0], acc[t][1], av[u], brow[t * 8]);
                     }
                 }
                 cp_async_wait_all();
                 __syncthreads();
             }
+            // the four lanes of a point hold the sums over facets q mod 4
 #pragma unroll
-            for (int i = 0; i < kMT; i++) {
-                // the four lanes of a point hold the sums over facets q mod 4
+            for (int o = 1; o <= 2; o <<= 1) {
+                br += __shfl_xor_sync(full, br, o);
+                s_cl += __shfl_xor_sync(full, s_cl, o);
+                s_cls += __shfl_xor_sync(full, s_cls, o);
+                if (kX1) x1 += __shfl_xor_sync(full, x1, o);
 #pragma unroll
-                for (int o = 1; o <= 2; o <<= 1) {
-                    br[i] += __shfl_xor_sync(full, br[i], o);
-                    s_cl[i] += __shfl_xor_sync(full, s_cl[i], o);
-                    s_cls[i] += __shfl_xor_sync(full, s_cls[i], o);
-                    if (kX1) x1[i] += __shfl_xor_sync(full, x1[i], o);
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        T[i][c] += __shfl_xor_sync(full, T[i][c], o);
-                        S[i][c] += __shfl_xor_sync(full, S[i][c], o);
-                    }
+                for (int c = 0; c < 3; c++) {
+                    T[c] += __shfl_xor_sync(full, T[c], o);
+                    S[c] += __shfl_xor_sync(full, S[c], o);
                 }
-                if (!act[i]) continue;
-                PointGeom G;
-                point_geometry(P, p[i], B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
-                const double sc = G.scale;
+            }
+            if (!act) continue;
+            PointGeom G;
+            point_geometry(P, p, B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
+            const double sc = G.scale;
 #pragma unroll
-                for (int t = 0; t < NT; t++)
+            for (int t = 0; t < NT; t++)
 #pragma unroll
-                    for (int jj = 0; jj < 2; jj++) {
-                        const int k = t * 8 + 2 * q + jj;
-                        if (k < C) Jt[(size_t)k * npad + p[i]] = sc * acc[i][t][jj];
-                    }
-                if (kX1 && q == 0) Jt[(size_t)(8 * NT) * npad + p[i]] = sc * x1[i];
-                if (q == 0) {
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        double v = 0;
-#pragma unroll
-                        for (int c = 0; c < 3; c++) v = fma(T[i][c], G.de[c][k], fma(S[i][c], G.de0[c][k], v));
-                        Jt[(size_t)(C + k) * npad + p[i]] = sc * v;
-                    }
-                    Jt[(size_t)(C + 3) * npad + p[i]] = br[i] * G.dphp[0];
-                    Jt[(size_t)(C + 4) * npad + p[i]] = br[i] * G.dphp[1];
-                    Jt[(size_t)(C + 5) * npad + p[i]] = br[i] * G.dphp[2];
-                    Jt[(size_t)(C + 6) * npad + p[i]] = sc * s_cl[i] * cl;
-                    Jt[(size_t)(C + 7) * npad + p[i]] = sc * s_cls[i];
-                    yt[p[i]] = br[i] * sc;
+                for (int jj = 0; jj < 2; jj++) {
+                    const int k = t * 8 + 2 * q + jj;
+                    if (k < C) Jt[(size_t)k * npad + p] = sc * acc[t][jj];
                 }
+            if (kX1 && q == 0) Jt[(size_t)(8 * NT) * npad + p] = sc * x1;
+            if (q == 0) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    double v = 0;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) v = fma(T[c], G.de[c][k], fma(S[c], G.de0[c][k], v));
+                    Jt[(size_t)(C + k) * npad + p] = sc * v;
+                }
+                Jt[(size_t)(C + 3) * npad + p] = br * G.dphp[0];
+                Jt[(size_t)(C + 4) * npad + p] = br * G.dphp[1];
+                Jt[(size_t)(C + 5) * npad + p] = br * G.dphp[2];
+                Jt[(size_t)(C + 6) * npad + p] = sc * s_cl * cl;
+                Jt[(size_t)(C + 7) * npad + p] = sc * s_cls;
+                yt[p] = br * sc;
             }
         }
     }
@@ -912,11 +913,11 @@ __device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, i
 // 261 out of line; 253 with the halves balanced (ref_halves; one facet: 286,
 // four: 276, which need more than 128 registers).  With few coefficients four
 // fit: 500 points and 16 coefficients, 140 fits and 400: 112 -> 109 ms.
-// `p`: the thread's point, -1 for none.  want_cl, all: also the columns of the
+// `p`: the thread's point, -1 for none.  first: also the facet sums.  want_cl, all: also the columns of the
 // Lambert coefficient, of the (never fitted) Lommel-Seeliger one.
 template <int NCB, int H, int kFirst, int kCount>
-__device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool want_cl, bool all, double* Jt,
-                                      double* yt) {
+__device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool first, bool want_cl, bool all,
+                                      double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const DevProblem& P = *Pp;
     const Layout L = make_layout(P);
@@ -961,6 +962,10 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
 #pragma unroll
     for (int k = 0; k < kCount; k++) acc[k] = 0;
     double a0 = 0, a1 = 0, a2 = 0;  // H = 0: br, rot0, rot1; H = 1: s_cl, rot2, s_cls
+    constexpr int kSums = (4 + 3 * NCB + kThreads - 1) / kThreads;
+    double fsum[kSums];
+#pragma unroll
+    for (int u = 0; u < kSums; u++) fsum[u] = 0;
     for (int f0 = 0; f0 < F; f0 += kFch) {
         const int nf = min(kFch, F - f0);
         __syncthreads();
@@ -977,6 +982,27 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
             s_fac[ff * 5 + 4] = fa[3];
         }
         __syncthreads();
+        if (first) {
+            // the facet sums from the staged chunk, one thread per sum, facets in
+            // order: chck (conv.c:22-27), the facet-area sum
+            // (period_search_BOINC.cpp:900-902), the conv-row shape derivatives
+#pragma unroll
+            for (int u = 0; u < kSums; u++) {
+                const int job = tid + u * kThreads;
+                if (job >= 4 + 3 * C) continue;
+                double s = fsum[u];
+                if (job < 3) {
+                    for (int ff = 0; ff < nf; ff++) s = s + s_fac[ff * 5 + 3] * s_fac[ff * 5 + job];
+                } else if (job == 3) {
+                    for (int ff = 0; ff < nf; ff++) s = s + s_fac[ff * 5 + 3];
+                } else {
+                    const int nc = (job - 4) / C, j = (job - 4) - nc * C;
+#pragma unroll 4
+                    for (int ff = 0; ff < nf; ff++) s += s_fac[ff * 5 + 4] * s_dg[ff * NCB + j] * s_fac[ff * 5 + nc];
+                }
+                fsum[u] = s;
+            }
+        }
         // kU facets at a time: their per-pair terms without a branch, side by side,
         // then the sums, facet by facet
         for (int f1 = 0; f1 < nf; f1 += kU) {
@@ -1031,6 +1057,17 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
             }
         }
     }
+    if (first) {
+        double* dres = sm + L.dres;
+#pragma unroll
+        for (int u = 0; u < kSums; u++) {
+            const int job = tid + u * kThreads;
+            if (job < 4)
+                sm[L.misc + (job < 3 ? M_CHK0 + job : M_SAREA)] = fsum[u];
+            else if (job < 4 + 3 * C)
+                dres[job - 4] = fsum[u];
+        }
+    }
     if (act) {
         PointGeom G;  // recomputed (the same values): no registers across the facet loop
         point_geometry(P, p, B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
@@ -1057,13 +1094,13 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
 // derivative and brightness sum are 17 operations per pair, the shape sums 2
 // each, so half 1 takes eight more of them.
 template <int NCB, int kTotal>
-__device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool want_cl, bool all,
-                                           double* Jt, double* yt) {
+__device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool first, bool want_cl,
+                                           bool all, double* Jt, double* yt) {
     constexpr int k0 = kTotal > 9 ? (kTotal - 8) / 2 & ~1 : 0;  // even: dg is read in pairs
     if (h == 0)
-        ref_pass<NCB, 0, 0, k0>(Pp, p, want_cl, all, Jt, yt);
+        ref_pass<NCB, 0, 0, k0>(Pp, p, first, want_cl, all, Jt, yt);
     else
-        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, want_cl, all, Jt, yt);
+        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, first, want_cl, all, Jt, yt);
 }
 
 // ref_pass over every data point, in segments sorted by viewing direction.
@@ -1084,11 +1121,12 @@ __device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp
         sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
         for (int base = 0; base < seg; base += kPts) {
             const int p = base + pl < seg ? perm[base + pl] : -1;
+            const bool first = s0 == 0 && base == 0;
             // C = 1 mod 8 for every even lmax = mmax: no sums for the padding
             if (P.C > NCB - 7)
-                ref_halves<NCB, NCB>(Pp, h, p, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB>(Pp, h, p, first, want_cl, all, Jt, yt);
             else
-                ref_halves<NCB, NCB - 7>(Pp, h, p, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB - 7>(Pp, h, p, first, want_cl, all, Jt, yt);
         }
     }
 }
@@ -1211,39 +1249,14 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
     eval_scalars(a, C, B, D, misc);
     curv_phase(P, a, g, area);
     __syncthreads();
-    // Sequential facet sums: chck / conv residuals (conv.c:22-27), the
-    // facet-area sum (period_search_BOINC.cpp:900-902) and the conv-row shape
-    // derivatives, one thread per sum, facets in order (the fast form forms
-    // them from the facet chunks its point loop stages).
-    if constexpr (!kFast)
-    for (int job = tid; job < 4 + 3 * C; job += kThreads) {
-        double s = 0;
-        if (job < 3) {
-#pragma unroll 8
-            for (int f = 0; f < F; f++) s = s + area[f] * P.fac[(size_t)f * 4 + job];
-            misc[M_CHK0 + job] = s;
-        } else if (job == 3) {
-#pragma unroll 8
-            for (int f = 0; f < F; f++) s = s + area[f];
-            misc[M_SAREA] = s;
-        } else {
-            const int nc = (job - 4) / C, j = (job - 4) - nc * C;
-#pragma unroll 8
-            for (int f = 0; f < F; f++) {
-                const double dg = g[f] * P.dsph[(size_t)f * NCB + j];
-                s += P.fac[(size_t)f * 4 + 3] * dg * P.fac[(size_t)f * 4 + nc];
-            }
-            dres[nc * C + j] = s;
-        }
-    }
     if constexpr (kFast) {
         if constexpr (NCB >= 16) {
             if (C == NCB - 7)
-                point_loop_fast<NCB, true>(P, sm, L, B, D, misc, g, area, dres, work, Jt, yt);
+                point_loop_fast<NCB, true>(Pp, Jt, yt);
             else
-                point_loop_fast<NCB, false>(P, sm, L, B, D, misc, g, area, dres, work, Jt, yt);
+                point_loop_fast<NCB, false>(Pp, Jt, yt);
         } else {
-            point_loop_fast<NCB, false>(P, sm, L, B, D, misc, g, area, dres, work, Jt, yt);
+            point_loop_fast<NCB, false>(Pp, Jt, yt);
         }
     } else {
         point_loop_ref<NCB>(Pp, sm, L, all, Jt, yt);
