@@ -718,8 +718,10 @@ __device__ __forceinline__ void chi2_rows(const DevProblem& P, const double* yt,
 // facets at a time (model_facets).
 // Buffers (shared memory): g, area [F] (area is not padded past F here);
 // misc and B/D (blmatrix) as in evaluate(); work >= max(sortseg, 4 kMf,
-// kThreads) doubles, 16-byte aligned; perm sortseg ints.  Used by the FP64
-// fit kernels (evaluate_model) and the mixed-precision one.
+// kThreads) doubles, 16-byte aligned; perm sortseg ints.  sorted: perm still
+// holds the points in the order of a nearby viewing geometry (any order gives
+// the same sums).  Used by the FP64 fit kernels (evaluate_model) and the
+// mixed-precision one.
 // Facets [0, kU) of `nrm` ({nx, ny, nz, Area}, zeros where there is no facet)
 // for one point per lane: the terms of all kU without a branch, so that their
 // chains run side by side, then the sum in facet order.  A facet that the lane
@@ -768,7 +770,7 @@ __device__ __forceinline__ void model_facets(const double4* nrm, const double* e
 // on the way (four lanes of the last warp, facets in order).
 template <bool kFast, bool kPlain>
 __device__ __forceinline__ void model_points(const DevProblem& P, const double* area, double* misc, const double* B,
-                                             double* work, int* perm, double* yt) {
+                                             double* work, int* perm, bool sorted, double* yt) {
     constexpr int kU = 4;  // facets at a time
     const int tid = threadIdx.x, F = P.F, job = tid - (kThreads - 32);
     const double cl = misc[M_CL], cls = misc[M_CLS];
@@ -778,7 +780,7 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
     for (int s0 = 0; s0 < P.n_points; s0 += P.sortseg) {
         const int seg = min(P.sortseg, P.n_points - s0);
         __syncthreads();
-        sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
+        if (!sorted) sort_points(P, s0, seg, B, misc[M_OMG], (unsigned long long*)work, perm);
         // kMp points per thread at most (slot j of thread t: point base + j kThreads
         // + t, so each slot's warp holds consecutive sorted points)
         const int k = min(kMp, (seg + kThreads - 1) / kThreads);
@@ -843,16 +845,21 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
 
 template <bool kFast>
 __device__ void model_pass(const DevProblem& P, const double* a, double* g, double* area, double* misc, double* B,
-                           double* D, double* work, int* perm, double* yt) {
+                           double* D, double* work, int* perm, bool sorted, double* yt) {
     const int tid = threadIdx.x;
+    // perm holds one segment.  A trial point lies near the accepted one, so the
+    // order of its Jacobian pass serves (sorting took 50 000 of the pass's 600 000
+    // cycles at 760 points; kept for the whole fit, the point loop lost more:
+    // 260 ms against 249 for 600 fits in the reference-order form)
+    sorted = sorted && P.n_points <= P.sortseg;
     eval_scalars(a, P.C, B, D, misc);
     curv_phase(P, a, g, area, false);
     __syncthreads();
     const double cls = misc[M_CLS];
     if (kFast || (fabs(cls) > 1e-200 && fabs(cls) < 1e200))
-        model_points<kFast, true>(P, area, misc, B, work, perm, yt);
+        model_points<kFast, true>(P, area, misc, B, work, perm, sorted, yt);
     else
-        model_points<kFast, false>(P, area, misc, B, work, perm, yt);
+        model_points<kFast, false>(P, area, misc, B, work, perm, sorted, yt);
     __syncthreads();
     if (tid < 3) yt[P.n_points + tid] = misc[M_CHK0 + tid];
     // relative-lightcurve normalisation of the model, mrqcof.c:53-58, 92-104
@@ -885,14 +892,14 @@ __device__ void model_pass(const DevProblem& P, const double* a, double* g, doub
 // normals when they fit there (nothing reads them after the pass but its own
 // normalisation and chi2), else to yt in global memory.
 template <int NCB, bool kFast>
-__device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, int a_off, double* yt) {
+__device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, int a_off, bool sorted, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const DevProblem& P = *Pp;
     const Layout L = make_layout(P);
     const int yoff = P.sortseg > 4 * kMf ? P.sortseg : 4 * kMf;
     double* ym = yoff + P.npad <= L.wlen ? sm + L.work + yoff : yt;
     model_pass<kFast>(P, sm + a_off, sm + L.g, sm + L.area, sm + L.misc, sm + L.blm, sm + L.blm + 9, sm + L.work,
-                      (int*)(sm + L.perm), ym);
+                      (int*)(sm + L.perm), sorted, ym);
 }
 
 // bright.c:54-125 in the reference's operation order (PS_FORM_FP64) for a pass
@@ -1459,7 +1466,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
                     atry[l] = cg[l] + da[j];
                 }
                 __syncthreads();
-                evaluate_model<NCB, kFast>(Pp, (int)(atry - sm), yt);
+                evaluate_model<NCB, kFast>(Pp, (int)(atry - sm), true, yt);
                 const double temp = misc[M_CHISQ];
                 chisq = temp;
                 s_last = misc[M_SAREA];

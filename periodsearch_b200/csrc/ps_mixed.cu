@@ -642,7 +642,7 @@ __device__ __noinline__ void evaluate_model_mixed(const DevProblem* __restrict__
     const size_t y_off = (work_off + (size_t)model_work_doubles(P) * 8 + (size_t)P.sortseg * 4 + 15) & ~(size_t)15;
     double* ym = y_off + (size_t)P.npad * 8 <= (size_t)(4 * kTileP * 128 + 4 * kNc * 128) ? (double*)(M.base + y_off)
                                                                                            : yt;
-    fitimpl::model_pass<true>(P, a, g, M.d(L.area), M.d(L.misc), M.d(L.blm), M.d(L.blm) + 9, work, perm, ym);
+    fitimpl::model_pass<true>(P, a, g, M.d(L.area), M.d(L.misc), M.d(L.blm), M.d(L.blm) + 9, work, perm, false, ym);
 }
 
 __device__ void tmem_setup(const DevProblem& P, uint8_t* raw, uint32_t* tmem) {
