@@ -259,11 +259,11 @@ int ps_chi2_grad(ps_ctx* ctx, const double* a, double* chi2, double* beta);
 int ps_gn_product(ps_ctx* ctx, const double* a, const double* v, double* out);
 /* One LM fit as ps_fit (period_search_BOINC.cpp:817-920; mrqmin.c:11-110
  * with gauss_errc's full pivoting), Jacobian-free: every model evaluation
- * runs the matrix-free kernels, alpha column by column from mfit
- * Gauss-Newton products with the free unit vectors, beta and chi2 from the
+ * runs the matrix-free kernels, alpha from mfit Gauss-Newton products with
+ * the free unit vectors, eight at a time, beta and chi2 from the
  * gradient pass, the trial points from the gradient pass alone, and the
  * solve on the host in FP64.  J is never formed (for shapes whose N x ma
- * Jacobian would not fit); each accepted step costs mfit + 1 matrix-free
+ * Jacobian would not fit); each accepted step costs mfit / 8 + 1 matrix-free
  * passes over the whole GPU, so for shapes whose J fits, ps_fit and the
  * scans are far faster.  Same outputs as ps_fit, up to rounding. */
 int ps_fit_jfree(ps_ctx* ctx, double freq, int pole, ps_fit_result* out, double* cg_out);

@@ -1,6 +1,7 @@
 // Matrix-free derivatives of the convex-inversion model (PS_FORM_FAST
 // arithmetic, FP64): chi2 and beta = J^T W (y_obs - y) -- the chi2 gradient is
-// -2 beta -- and the Gauss-Newton product J^T W (J v), without forming J.
+// -2 beta -- and Gauss-Newton products J^T W (J v), one or kAdjDirs at a time,
+// without forming J.
 //
 // The shape block of J is J_pk = Scale_p sum_f Darea_f s_pf g_f Dsph_fk
 // (bright.c:78-85 with Dg = g Dsph, curv.c:31-35).  Its products with a vector
@@ -9,23 +10,23 @@
 //   (J^T l)_k = sum_f (sum_p l_p Scale_p s_pf) Area_f Dsph_fk       (adjoint)
 // so one product costs two passes over the (point, facet) pairs plus two
 // F x C contractions instead of the N F C of the explicit Jacobian.  The eight
-// non-shape columns are formed per point.  The relative-lightcurve
-// normalisation (mrqcof.c:92-104), J'_r = coef (J_r - y_r dave / ave) with
-// dave = sum_r J_r and J'_r1 = 0, becomes per-lightcurve scalars:
+// non-shape columns are formed per point, and so is the first shape column:
+// Dsph_f0 = 1, so it is the model itself, and z leaves the first coefficient
+// out.  The relative-lightcurve normalisation (mrqcof.c:92-104),
+// J'_r = coef (J_r - y_r dave / ave) with dave = sum_r J_r and J'_r1 = 0,
+// becomes per-lightcurve scalars:
 //   (J' v)_r  = coef ((J v)_r - y_r sum_{r'} (J v)_{r'} / ave)   (v_1 left out)
 //   J'^T u    = J^T l,  l_r = coef (u_r - sum_{r'} y_{r'} u_{r'} / ave).
-// The convexity rows (conv.c:12-29) are added explicitly.  Every reduction
-// runs in a fixed order, so results are deterministic.
+// A convexity row (conv.c:12-29) is a point whose s_pf is a component of the
+// facet's normal, so its weights join the facet sums.  Every reduction runs in
+// a fixed order, so results are deterministic.
 //
-// Kernels, in stream order, each spread over the GPU: adj_curv (thread per
-// facet: blmatrix, curv, z), adj_conv (warp per convexity-row sum),
-// adj_points (thread per point and facet slice), adj_points_fin (thread per
-// point: the slices' sums in order, the per-point results), adj_lc (CTA per lightcurve: model and J v
-// sums), adj_rowsum (rows: normalised model, residual, u, per-CTA chi2),
-// adj_lck (CTA per lightcurve: the adjoint's y.u sum), adj_weights (thread
-// per point), adj_facets (thread per facet, blocks of points), adj_qs
-// (thread per facet), adj_cols (CTA per output column: the F x C
-// contraction and the non-shape columns), adj_out (the free parameters).
+// Six kernels, each spread over the GPU by how many CTAs its sizes give:
+// adj_curv (warp per facet: scalars, areas, z, facet sums), adj_points (point
+// blocks x facet slices), adj_rows (CTA per relative lightcurve or block of
+// calibrated points: the slices' sums, model, residual, adjoint weights),
+// adj_facets (facet blocks x point blocks), adj_cols (blocks of facets: the
+// F x C contraction), adj_out (CTA per free parameter).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -38,26 +39,64 @@ namespace {
 
 using namespace fitcommon;
 
-constexpr int kPtThreads = 128;  // adj_points: points per CTA
-constexpr int kFacetChunk = 256; // adj_points: facets staged per chunk
-constexpr int kFcThreads = 128;  // adj_facets: facets per CTA
-constexpr int kPtBlock = 512;    // adj_facets: points per CTA (staged)
-constexpr int kRowThreads = 256; // adj_rowsum: rows per CTA
-constexpr int kPart = 11;        // adj_points: partial sums per point and facet slice
-constexpr int kMaxSlices = 8;    // adj_points: facet slices at most
-
-// Facet slices of the (point, facet) pass: enough CTAs to fill the GPU,
-// slices of at least 256 facets.
-inline int facet_slices(const DevProblem& P) {
-    const int pb = (P.n_points + kPtThreads - 1) / kPtThreads;
-    int s = 1;
-    while (s < kMaxSlices && pb * s < 4 * 148 && P.F / (2 * s) >= 256) s *= 2;
-    return s;
-}
+constexpr int kCurvFacets = 8;    // adj_curv: facets per CTA (a warp each)
+constexpr int kPtThreads = 128;   // adj_points: points per CTA
+constexpr int kPairChunk = 64;    // adj_points: facet pairs staged at a time
+constexpr int kRowThreads = kAdjRowBlock;  // adj_rows
+constexpr int kFcThreads = 128;   // adj_facets: facets per CTA
+constexpr int kPtStage = 64;      // adj_facets: points staged at a time
+constexpr int kColFacets = 32;    // adj_cols: facets per CTA
+constexpr int kFixed = 9;         // adj_points: sums besides the directions'
+constexpr int kMaxSlices = 32;    // adj_points: facet slices at most
+constexpr int kMaxPointBlocks = 64;  // adj_facets: point blocks at most
+constexpr int kFill = 4 * 148;    // CTAs that fill the GPU
 
 // misc slots (X_CHK and X_SAREA are read by the host: kAdjMiscChk, kAdjMiscSarea)
 enum { X_B = 0, X_D = 9, X_CL = 27, X_CLS = 28, X_OMG = 29, X_P1 = 30, X_P2 = 31, X_P3 = 32, X_CHK = kAdjMiscChk,
-       X_SAREA = kAdjMiscSarea, X_N = 40 };
+       X_SAREA = kAdjMiscSarea, X_UC = 40, X_N = X_UC + 3 * kAdjDirs };
+
+// Device work arrays of one evaluation, carved from one buffer of
+// adjoint_work_doubles(P) doubles; K directions.
+struct AdjWork {
+    double* misc;    // scalars, then u of the convexity rows [K][3]
+    double* dir;     // [K][9]: v of the first shape coefficient, then of the non-shape parameters
+    double* area;    // [F]
+    double* z;       // [K][F]
+    double* cpart;   // [4 + 3 K][curv CTAs]: chck, area sum, J v of the convexity rows
+    double* e6;      // [6][N]: e, e0
+    double* pp;      // [kFixed + K][nfs][N]
+    double* jns;     // [9][N]: non-shape columns, first shape column (0 on relative rows)
+    double *y, *scale;  // [N]
+    double* jv;      // [K][N]
+    double* lam;     // [K][N] adjoint weights
+    double* ls;      // [K][N] times Scale
+    double* x2part;  // [row items]
+    double* q;       // [K][npb][F]
+    double* cols;    // [K][col CTAs][C]
+    double* out;     // [K][mfit]
+    double* chi2;
+    int nfs, npb, ppb;  // facet slices; point blocks and their points
+    int ncurv, ncol;
+    AdjMode mode;
+};
+
+inline int cdiv(int a, int b) { return (a + b - 1) / b; }
+
+// Facet slices of adj_points: enough CTAs to fill the GPU, 16 pairs or more.
+inline int facet_slices(const DevProblem& P) {
+    const int blocks = cdiv(P.n_points, kPtThreads);
+    int s = cdiv(kFill, blocks);
+    if (s > P.F / 2 / 16) s = P.F / 2 / 16;
+    return s < 1 ? 1 : s > kMaxSlices ? kMaxSlices : s;
+}
+
+// Points per CTA of adj_facets: likewise, 32 or more.
+inline int points_per_block(const DevProblem& P) {
+    int blocks = cdiv(kFill, cdiv(P.F, kFcThreads));
+    if (blocks > kMaxPointBlocks) blocks = kMaxPointBlocks;
+    const int n = cdiv(P.n_points, blocks);
+    return n < 32 ? 32 : n;
+}
 
 __device__ double block_sum(double v, double* red) {
     // fixed-order tree: warp shuffles, then warp 0 over the warp partials
@@ -78,447 +117,485 @@ __device__ double block_sum(double v, double* red) {
     return s;
 }
 
-// blmatrix and the scattering/phase scalars (block 0), curv (curv.c:15-37)
-// and z = Dsph v, z0 = z without the first coefficient; thread per facet.
-__global__ void adj_curv(const DevProblem* __restrict__ Pp, AdjWork W) {
+__device__ __forceinline__ double warp_sum(double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// 1 / d for d in (2e-8, 2], correctly rounded but for a handful of operands:
+// the hardware's approximation, a cubic and a Newton step.  No branch.
+__device__ __forceinline__ double recip(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    double e = fma(-d, r, 1.0);
+    r = fma(r, fma(e, e, e), r);
+    e = fma(-d, r, 1.0);
+    return fma(r, e, r);
+}
+
+// blmatrix, the scattering and phase scalars and the directions' non-shape
+// parts (block 0); curv (curv.c:15-37 through Dsph = Fc/Fs Pleg), z without the
+// first coefficient, and each CTA's share of the facet sums: a warp per facet,
+// lanes over the coefficients.  (A thread per facet read its rows uncoalesced:
+// 26 us at 2048 facets and 81 coefficients.)
+template <int K>
+__global__ void __launch_bounds__(32 * kCurvFacets) adj_curv(const DevProblem* __restrict__ Pp, AdjWork W, const AdjArgs A) {
     const DevProblem& P = *Pp;
-    const double* a = W.a;
-    const int C = P.C, NCB = P.NCB;
-    double* x = W.misc;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        blmatrix(a[C], a[C + 1], x + X_B, x + X_D);
-        x[X_CL] = exp(a[C + 6]);
-        x[X_CLS] = a[C + 7];
-        x[X_OMG] = a[C + 2];
-        x[X_P1] = a[C + 3];
-        x[X_P2] = a[C + 4];
-        x[X_P3] = a[C + 5];
-    }
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= P.F) return;
-    const double* pl = P.cpl + (size_t)f * P.nq;
-    const double* fc = P.cfc + (size_t)f * (P.mmax + 1);
-    const double* fs = P.cfs + (size_t)f * (P.mmax + 1);
-    double gi = 0;
-    int n = 0, q = 0;
-    for (int m = 0; m <= P.mmax; m++) {
-        for (int l = m; l <= P.lmax; l++) {
-            double fsum = a[n] * fc[m];
-            n++;
-            if (m != 0) {
-                fsum = fma(a[n], fs[m], fsum);
-                n++;
-            }
-            gi = fma(pl[q], fsum, gi);
-            q++;
+    const int C = P.C, F = P.F, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ double part[4 + 3 * K][kCurvFacets];
+    if (blockIdx.x == 0) {
+        double* x = W.misc;
+        if (tid == 0) {
+            blmatrix(A.a[C], A.a[C + 1], x + X_B, x + X_D);
+            x[X_CL] = exp(A.a[C + 6]);
+            x[X_CLS] = A.a[C + 7];
+            x[X_OMG] = A.a[C + 2];
+            x[X_P1] = A.a[C + 3];
+            x[X_P2] = A.a[C + 4];
+            x[X_P3] = A.a[C + 5];
+        }
+        for (int i = tid; i < 9 * K; i += blockDim.x) {
+            const int d = i / 9, j = i - 9 * d, k = j == 0 ? 0 : C + j - 1;
+            W.dir[i] = W.mode == kAdjUnits ? (A.unit[d] == k ? 1.0 : 0.0) : W.mode == kAdjProduct ? A.v[k] : 0.0;
         }
     }
-    gi = exp(gi);
-    W.g[f] = gi;
-    W.area[f] = P.fac[(size_t)f * 4 + 3] * gi;
-    double z = 0;
-    const double* ds = P.dsph + (size_t)f * NCB;
-    if (W.v)
-        for (int k = 1; k < C; k++) z = fma(ds[k], W.v[k], z);
-    W.z0[f] = z;
-    W.z[f] = W.v ? fma(ds[0], W.v[0], z) : 0.0;
-}
-
-// Convexity rows: chck_nc = sum Area n_nc and dres_nc,k = sum Darea g Dsph_k
-// n_nc, and the facet-area sum; one warp per sum (lanes stride the facets,
-// fixed-order shuffle tree).
-__global__ void adj_conv(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    const int F = P.F, C = P.C, NCB = P.NCB;
-    const int job = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (job >= 4 + 3 * C) return;
-    double s = 0;
-    if (job < 3) {
-        for (int f = lane; f < F; f += 32) s = fma(W.area[f], P.fac[(size_t)f * 4 + job], s);
-    } else if (job == 3) {
-        for (int f = lane; f < F; f += 32) s += W.area[f];
-    } else {
-        const int nc = (job - 4) / C, k = (job - 4) - nc * C;
-        for (int f = lane; f < F; f += 32) s = fma(W.area[f] * P.dsph[(size_t)f * NCB + k], P.fac[(size_t)f * 4 + nc], s);
+    const int f = blockIdx.x * kCurvFacets + warp;
+    double x = 0, z[K], n[3] = {0, 0, 0}, area = 0;
+#pragma unroll
+    for (int d = 0; d < K; d++) z[d] = 0;
+    if (f < F) {
+        const double* ds = P.dsph + (size_t)f * P.NCB;
+        for (int k = lane; k < C; k += 32) {
+            const double b = ds[k];
+            x = fma(A.a[k], b, x);
+            if (K == 1 && W.mode == kAdjProduct && k > 0) z[0] = fma(A.v[k], b, z[0]);
+        }
+        x = warp_sum(x);
+        if (K == 1) z[0] = warp_sum(z[0]);
+        if constexpr (K > 1) {
+#pragma unroll
+            for (int d = 0; d < K; d++) {
+                const int k = A.unit[d];
+                z[d] = k > 0 && k < C ? ds[k] : 0.0;
+            }
+        }
+        const double* fa = P.fac + (size_t)f * 4;
+        area = fa[3] * exp(x);
+        for (int c = 0; c < 3; c++) n[c] = fa[c];
+        if (lane == 0) {
+            W.area[f] = area;
+#pragma unroll
+            for (int d = 0; d < K; d++) W.z[(size_t)d * F + f] = z[d];
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) {
-        if (job < 3)
-            W.misc[X_CHK + job] = s;
-        else if (job == 3)
-            W.misc[X_SAREA] = s;
-        else
-            W.dres[job - 4] = s;
+        for (int c = 0; c < 3; c++) part[c][warp] = area * n[c];
+        part[3][warp] = area;
+#pragma unroll
+        for (int d = 0; d < K; d++) {
+            double v0 = 0;
+            if (W.mode == kAdjUnits) v0 = A.unit[d] == 0 ? 1.0 : 0.0;
+            if (W.mode == kAdjProduct) v0 = A.v[0];
+            for (int c = 0; c < 3; c++) part[4 + 3 * d + c][warp] = area * n[c] * (z[d] + v0);
+        }
+    }
+    __syncthreads();
+    if (tid < 4 + 3 * K) {
+        double s = 0;
+        for (int w = 0; w < kCurvFacets; w++) s += part[tid][w];
+        W.cpart[(size_t)tid * W.ncurv + blockIdx.x] = s;
     }
 }
 
-// Per point and facet slice: partial sums over the slice's facets of the
-// model brightness and of what the eight non-shape columns and the shape
-// part of J v need (br, Area s z, Area s z0, the Lambert / Lommel-Seeliger
-// sums, T = sum Area dsmu n, S = sum Area dsmu0 n); grid (point blocks,
-// facet slices), so that the (point, facet) pass fills the GPU.
+// Per point and facet slice: the slice's sums of the model brightness and of
+// what the non-shape columns and the shape parts of J v need (Area s z per
+// direction, the Lambert / Lommel-Seeliger sums, T = sum Area dsmu n,
+// S = sum Area dsmu0 n); grid (point blocks, facet slices).  Facets come in
+// antipodal pairs, of which a point sees at most one: an FP32 cosine picks the
+// side, so a warp's lanes work on a facet they see in nine of ten pairs, where
+// facet by facet 45 % of the lanes were active and points in time order share
+// no facets to skip (20 000 points, 2048 facets: 174 us).  Where the FP32 sign
+// is wrong (a facet within 1e-6 of grazing) the pair's two facets are tested in
+// FP64.
+template <int K>
 __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
-    __shared__ double sf[6][kFacetChunk];  // nx, ny, nz, Area, z, z0
+    __shared__ double sf[4 + K][2 * kPairChunk];  // nx, ny, nz, Area, z; [pair][side]
     const int tid = threadIdx.x, F = P.F, N = P.n_points;
     const int p = blockIdx.x * kPtThreads + tid;
     const bool act = p < N;
-    const int per = (F + W.nfs - 1) / W.nfs;
-    const int fa0 = blockIdx.y * per, fa1 = min(F, fa0 + per);
+    const int pairs = F / 2, per = (pairs + W.nfs - 1) / W.nfs;
+    const int j0 = blockIdx.y * per, j1 = min(pairs, j0 + per);
     const double* x = W.misc;
     const double cl = x[X_CL], cls = x[X_CLS];
-    PointGeom G;
-    if (act) point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
-    double acc[kPart] = {};
-    for (int f0 = fa0; f0 < fa1; f0 += kFacetChunk) {
-        const int nf = min(kFacetChunk, fa1 - f0);
+    double e[3] = {0, 0, 0}, e0[3] = {0, 0, 0};
+    if (act) {
+        PointGeom G;
+        point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
+        for (int c = 0; c < 3; c++) {
+            e[c] = G.e[c];
+            e0[c] = G.e0[c];
+            if (blockIdx.y == 0) {
+                W.e6[(size_t)c * N + p] = e[c];
+                W.e6[(size_t)(3 + c) * N + p] = e0[c];
+            }
+        }
+    }
+    const float e32[3] = {(float)e[0], (float)e[1], (float)e[2]};
+    double acc[kFixed + K] = {};
+    for (int c0 = j0; c0 < j1; c0 += kPairChunk) {
+        const int np = min(kPairChunk, j1 - c0);
         __syncthreads();
-        for (int i = tid; i < nf; i += kPtThreads) {
-            const double* fa = P.fac + (size_t)(f0 + i) * 4;
+        for (int i = tid; i < 2 * np; i += kPtThreads) {
+            const int f = P.apair[2 * c0 + i];
+            const double* fa = P.fac + (size_t)f * 4;
             sf[0][i] = fa[0];
             sf[1][i] = fa[1];
             sf[2][i] = fa[2];
-            sf[3][i] = W.area[f0 + i];
-            sf[4][i] = W.z[f0 + i];
-            sf[5][i] = W.z0[f0 + i];
+            sf[3][i] = W.area[f];
+#pragma unroll
+            for (int d = 0; d < K; d++) sf[4 + d][i] = W.z[(size_t)d * F + f];
         }
         __syncthreads();
-        if (!act) continue;
-        for (int i = 0; i < nf; i++) {
-            const double nx = sf[0][i], ny = sf[1][i], nz = sf[2][i];
-            const double mu = G.e[0] * nx + G.e[1] * ny + G.e[2] * nz;
-            const double mu0 = G.e0[0] * nx + G.e0[1] * ny + G.e0[2] * nz;
-            if (mu > kTinyD && mu0 > kTinyD) {
-                const double ar = sf[3][i];
-                const double r = 1.0 / (mu + mu0);
-                const double s = mu * mu0 * fma(cls, r, cl);
-                const double t = ar * s;
-                acc[0] += t;                      // br
-                acc[1] = fma(t, sf[4][i], acc[1]);  // sum Area s z
-                acc[2] = fma(t, sf[5][i], acc[2]);  // sum Area s z0
-                const double q0 = mu0 * r, q1 = mu * r;
-                const double w = ar * fma(cls * q0, q0, cl * mu0);
-                const double w0 = ar * fma(cls * q1, q1, cl * mu);
-                acc[3] = fma(w, nx, acc[3]);
-                acc[4] = fma(w, ny, acc[4]);
-                acc[5] = fma(w, nz, acc[5]);
-                acc[6] = fma(w0, nx, acc[6]);
-                acc[7] = fma(w0, ny, acc[7]);
-                acc[8] = fma(w0, nz, acc[8]);
-                const double mm = mu * mu0 * ar;
-                acc[9] += mm;                     // sum mu mu0 Area
-                acc[10] = fma(mm, r, acc[10]);    // sum mu mu0 Area / (mu + mu0)
+#pragma unroll 2
+        for (int j = 0; j < np; j++) {
+            const float m32 = e32[0] * (float)sf[0][2 * j] + e32[1] * (float)sf[1][2 * j] + e32[2] * (float)sf[2][2 * j];
+            int i = 2 * j + (m32 < 0.f);
+            double nx = sf[0][i], ny = sf[1][i], nz = sf[2][i];
+            double mu = fma(e[2], nz, fma(e[1], ny, e[0] * nx));
+            if (mu < 0) {  // the other side after all
+                i ^= 1;
+                nx = sf[0][i], ny = sf[1][i], nz = sf[2][i];
+                mu = fma(e[2], nz, fma(e[1], ny, e[0] * nx));
             }
+            const double mu0 = fma(e0[2], nz, fma(e0[1], ny, e0[0] * nx));
+            const bool vis = mu > kTinyD && mu0 > kTinyD;
+            const double ar = vis ? sf[3][i] : 0.0;
+            const double r = recip(vis ? mu + mu0 : 1.0);
+            const double am = ar * mu, am0 = ar * mu0, mm = am * mu0, cr = cls * r, crr = cr * r;
+            const double t = mm * (cr + cl);
+            acc[0] += t;                      // br
+            acc[1] += mm;                     // sum mu mu0 Area
+            acc[2] = fma(mm, r, acc[2]);      // sum mu mu0 Area / (mu + mu0)
+            const double w = am0 * fma(crr, mu0, cl), w0 = am * fma(crr, mu, cl);
+            acc[3] = fma(w, nx, acc[3]);
+            acc[4] = fma(w, ny, acc[4]);
+            acc[5] = fma(w, nz, acc[5]);
+            acc[6] = fma(w0, nx, acc[6]);
+            acc[7] = fma(w0, ny, acc[7]);
+            acc[8] = fma(w0, nz, acc[8]);
+#pragma unroll
+            for (int d = 0; d < K; d++) acc[kFixed + d] = fma(t, sf[4 + d][i], acc[kFixed + d]);
         }
     }
     if (!act) return;
-    for (int j = 0; j < kPart; j++) W.pp[((size_t)j * W.nfs + blockIdx.y) * N + p] = acc[j];
+#pragma unroll
+    for (int j = 0; j < kFixed + K; j++) W.pp[((size_t)j * W.nfs + blockIdx.y) * N + p] = acc[j];
 }
 
-// Per point: the slices' partial sums in slice order, then the model, the
-// eight non-shape columns of J, the shape part of J v (with and without the
-// first coefficient), Scale, and e, e0 for the adjoint pass.
-__global__ void adj_points_fin(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    const int N = P.n_points, C = P.C;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= N) return;
-    const double* x = W.misc;
-    const double cl = x[X_CL];
-    PointGeom G;
-    point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
-    double acc[kPart];
-    for (int j = 0; j < kPart; j++) {
-        double v = 0;
-        for (int k = 0; k < W.nfs; k++) v += W.pp[((size_t)j * W.nfs + k) * N + p];
-        acc[j] = v;
-    }
-    const double br = acc[0], sz = acc[1], sz0 = acc[2], s_cl = acc[9], s_cls = acc[10];
-    const double sc = G.scale;
-    double jn[8];
-    const double T[3] = {acc[3], acc[4], acc[5]}, S[3] = {acc[6], acc[7], acc[8]};
-    for (int k = 0; k < 3; k++) {
-        double v = 0;
-        for (int j = 0; j < 3; j++) v = fma(T[j], G.de[j][k], fma(S[j], G.de0[j][k], v));
-        jn[k] = sc * v;
-    }
-    jn[3] = br * G.dphp[0];
-    jn[4] = br * G.dphp[1];
-    jn[5] = br * G.dphp[2];
-    jn[6] = sc * s_cl * cl;
-    jn[7] = sc * s_cls;
-    double ns = 0;
-    for (int j = 0; j < 8; j++) {
-        W.jns[(size_t)j * N + p] = jn[j];
-        if (W.v) ns = fma(jn[j], W.v[C + j], ns);
-    }
-    W.y[p] = br * sc;
-    W.scale[p] = sc;
-    W.jv[p] = fma(sc, sz, ns);
-    W.jv0[p] = fma(sc, sz0, ns);
-    for (int c = 0; c < 3; c++) {
-        W.e6[(size_t)c * N + p] = G.e[c];
-        W.e6[(size_t)(3 + c) * N + p] = G.e0[c];
-    }
-}
-
-// Lightcurve of data row r (binary search over the lightcurve starts).
-__device__ __forceinline__ int lc_of(const DevProblem& P, int r) {
-    int lo = 0, hi = P.n_lc - 2;  // the last lightcurve is the convexity pseudo-curve
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (P.lc_start[mid] <= r)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
-// Per relative lightcurve (one CTA each): ave = sum y, S = sum (J v without
-// v_1), coef = sig L / ave (mrqcof.c:53-58, 92-104).
-__global__ void adj_lc(const DevProblem* __restrict__ Pp, AdjWork W) {
+// One item of the row list per CTA: a relative lightcurve, a block of
+// calibrated points, or (the last) the three convexity rows.  Per point the
+// slices' sums in slice order, then the model, the non-shape columns of J and
+// J v; per relative lightcurve ave = sum y and S = sum J v without v_1
+// (mrqcof.c:53-58, 92-104); per row the normalised model and J v, the residual,
+// u = W (y_obs - y') or W J' v, and the item's share of chi2; the adjoint
+// weights l.  (Five kernels before: 45 us of launches and of passes over the
+// rows at 20 000 points.)
+template <int K>
+__global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
     __shared__ double red[32];
-    const int lc = blockIdx.x, nlc = P.n_lc - 1;
-    if (!P.lc_rel[lc]) return;
-    const int r0 = P.lc_start[lc], r1 = P.lc_start[lc + 1];
-    double sy = 0, sj = 0;
-    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-        sy += W.y[r];
-        sj += W.jv0[r];
-    }
-    sy = block_sum(sy, red);
-    sj = block_sum(sj, red);
-    if (threadIdx.x == 0) {
-        W.lcw[lc] = sy;
-        W.lcw[nlc + lc] = sj;
-        W.lcw[3 * nlc + lc] = P.sig[r0] * (double)P.lc_npts[lc] / sy;
-    }
-}
-
-// Rows: the normalised model and J v, the residual, u = W (y_obs - y') or
-// W J' v, and each CTA's share of chi2 (summed in block order by adj_cols).
-__global__ void adj_rowsum(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    __shared__ double red[32];
-    const int nlc = P.n_lc - 1;
-    const double* lc_ave = W.lcw;
-    const double* lc_s = W.lcw + nlc;
-    const double* lc_coef = W.lcw + 3 * nlc;
+    const int tid = threadIdx.x, N = P.n_points;
+    const int4 item = reinterpret_cast<const int4*>(P.arows)[blockIdx.x];  // first row, last + 1, relative, points of the curve
+    double* x = W.misc;
     double x2 = 0;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < P.n_rows) {
-        double yy, jv;
-        if (r < P.n_points) {
-            const int lc = lc_of(P, r);
-            if (P.lc_rel[lc]) {
-                const double coef = lc_coef[lc];
-                yy = coef * W.y[r];
-                jv = coef * (W.jv0[r] - W.y[r] * lc_s[lc] / lc_ave[lc]);
-            } else {
-                yy = W.y[r];
-                jv = W.jv[r];
+    if (item.x >= N) {
+        // the facet sums of adj_curv's CTAs, a warp per sum
+        const int lane = tid & 31;
+        for (int j = tid >> 5; j < 4 + 3 * K; j += kRowThreads / 32) {
+            double s = 0;
+            for (int b = lane; b < W.ncurv; b += 32) s += W.cpart[(size_t)j * W.ncurv + b];
+            s = warp_sum(s);
+            if (lane == 0) {
+                if (j < 4)
+                    x[X_CHK + j] = s;
+                else if (W.mode != kAdjGradient) {
+                    const int r = N + (j - 4) % 3;
+                    x[X_UC + j - 4] = P.sig2i[r] * P.wght[r] * s;
+                }
             }
-        } else {
-            // the convexity rows; their J v needs the C-term dot products
-            const int nc = r - P.n_points;
-            yy = W.misc[X_CHK + nc];
-            jv = 0;
-            if (W.v)
-                for (int k = 0; k < P.C; k++) jv = fma(W.dres[nc * P.C + k], W.v[k], jv);
         }
-        const double w = P.sig2i[r] * P.wght[r];
-        const double dy = P.yobs[r] - yy;
-        x2 = dy * dy * w;
-        W.u[r] = W.v ? w * jv : w * dy;
+        __syncthreads();
+        if (tid < 3) {
+            const int r = N + tid;
+            const double dy = P.yobs[r] - x[X_CHK + tid], w = P.sig2i[r] * P.wght[r];
+            x2 = dy * dy * w;
+            if (W.mode == kAdjGradient) x[X_UC + tid] = w * dy;
+        }
+        x2 = block_sum(x2, red);
+        if (tid == 0) W.x2part[blockIdx.x] = x2;
+        return;
+    }
+    const bool rel = item.z != 0;
+    const double cl = x[X_CL];
+    double sy = 0, sj[K];
+#pragma unroll
+    for (int d = 0; d < K; d++) sj[d] = 0;
+    for (int p = item.x + tid; p < item.y; p += kRowThreads) {
+        PointGeom G;
+        point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
+        double acc[kFixed + K];
+#pragma unroll
+        for (int j = 0; j < kFixed + K; j++) {
+            double v = 0;
+            for (int k = 0; k < W.nfs; k++) v += W.pp[((size_t)j * W.nfs + k) * N + p];
+            acc[j] = v;
+        }
+        const double br = acc[0], sc = G.scale, yy = br * sc;
+        double jn[9];
+        for (int k = 0; k < 3; k++) {
+            double v = 0;
+            for (int c = 0; c < 3; c++) v = fma(acc[3 + c], G.de[c][k], fma(acc[6 + c], G.de0[c][k], v));
+            jn[k] = sc * v;
+        }
+        jn[3] = br * G.dphp[0];
+        jn[4] = br * G.dphp[1];
+        jn[5] = br * G.dphp[2];
+        jn[6] = sc * acc[1] * cl;
+        jn[7] = sc * acc[2];
+        jn[8] = rel ? 0.0 : yy;  // first shape coefficient
+        for (int j = 0; j < 9; j++) W.jns[(size_t)j * N + p] = jn[j];
+        W.y[p] = yy;
+        W.scale[p] = sc;
+        sy += yy;
+#pragma unroll
+        for (int d = 0; d < K; d++) {
+            const double* v = W.dir + 9 * d;
+            double s = jn[8] * v[0];
+            for (int j = 0; j < 8; j++) s = fma(jn[j], v[1 + j], s);
+            s = fma(sc, acc[kFixed + d], s);
+            W.jv[(size_t)d * N + p] = s;
+            sj[d] += s;
+        }
+    }
+    double ave = 0, sjv[K], kap[K], coefn = 0;
+#pragma unroll
+    for (int d = 0; d < K; d++) sjv[d] = kap[d] = 0;
+    if (rel) {
+        ave = block_sum(sy, red);
+        coefn = (double)item.w / ave;
+#pragma unroll
+        for (int d = 0; d < K; d++) sjv[d] = block_sum(sj[d], red) / ave;
+    }
+    for (int p = item.x + tid; p < item.y; p += kRowThreads) {
+        const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0;
+        const double w = P.sig2i[p] * P.wght[p], dy = P.yobs[p] - coef * y;
+        x2 = fma(dy * w, dy, x2);
+#pragma unroll
+        for (int d = 0; d < K; d++) {
+            const double jv = W.jv[(size_t)d * N + p];
+            const double u = W.mode == kAdjGradient ? w * dy : w * (rel ? coef * (jv - y * sjv[d]) : jv);
+            W.lam[(size_t)d * N + p] = u;
+            kap[d] = fma(y, u, kap[d]);
+        }
+    }
+    if (rel) {
+#pragma unroll
+        for (int d = 0; d < K; d++) kap[d] = block_sum(kap[d], red) / ave;
+    }
+    for (int p = item.x + tid; p < item.y; p += kRowThreads) {
+        const double sc = W.scale[p], coef = rel ? P.sig[p] * coefn : 1.0;
+#pragma unroll
+        for (int d = 0; d < K; d++) {
+            double l = W.lam[(size_t)d * N + p];
+            if (rel) l = coef * (l - kap[d]);
+            W.lam[(size_t)d * N + p] = l;
+            W.ls[(size_t)d * N + p] = l * sc;
+        }
     }
     x2 = block_sum(x2, red);
-    if (threadIdx.x == 0) W.x2part[blockIdx.x] = x2;
+    if (tid == 0) W.x2part[blockIdx.x] = x2;
 }
 
-// Per relative lightcurve (one CTA each): kappa = sum y u / ave.
-__global__ void adj_lck(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    __shared__ double red[32];
-    const int lc = blockIdx.x, nlc = P.n_lc - 1;
-    if (!P.lc_rel[lc]) return;
-    const int r0 = P.lc_start[lc], r1 = P.lc_start[lc + 1];
-    double s = 0;
-    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) s = fma(W.y[r], W.u[r], s);
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) W.lcw[2 * nlc + lc] = s / W.lcw[lc];
-}
-
-// Adjoint weights per point: l (all columns), l0 (the first shape
-// coefficient, zero on relative rows); ls = l Scale for the facet pass.
-__global__ void adj_weights(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= P.n_points) return;
-    const int nlc = P.n_lc - 1;
-    const int lc = lc_of(P, r);
-    double l = W.u[r], l0 = l;
-    if (P.lc_rel[lc]) {
-        l = W.lcw[3 * nlc + lc] * (W.u[r] - W.lcw[2 * nlc + lc]);
-        l0 = 0.0;
-    }
-    W.lam[r] = l;
-    W.ls[r] = l * W.scale[r];
-    W.ls0[r] = l0 * W.scale[r];
-}
-
-// q_f = sum_p ls_p s_pf and q0_f = sum_p ls0_p s_pf over a block of points;
-// thread per facet, points staged in shared memory.
+// q_f = sum_p ls_p s_pf over a block of points; thread per facet (neighbours
+// see nearly the same points), points staged in shared memory, two points at a
+// time without a branch.  Blocks of points small enough to fill the GPU: in
+// blocks of 512, 760 points and 800 facets made 14 CTAs and 62 us.
+template <int K>
 __global__ void __launch_bounds__(kFcThreads) adj_facets(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
-    __shared__ double sp[8][kPtBlock];  // e (3), e0 (3), ls, ls0
-    const int f = blockIdx.x * kFcThreads + threadIdx.x;
-    const int p0 = blockIdx.y * kPtBlock;
-    const int np = min(kPtBlock, P.n_points - p0);
-    for (int i = threadIdx.x; i < np; i += kFcThreads) {
-        for (int c = 0; c < 6; c++) sp[c][i] = W.e6[(size_t)c * P.n_points + p0 + i];
-        sp[6][i] = W.ls[p0 + i];
-        sp[7][i] = W.ls0[p0 + i];
+    constexpr int kU = 2;
+    __shared__ double sp[6 + K][kPtStage];  // e (3), e0 (3), ls
+    const int f = blockIdx.x * kFcThreads + threadIdx.x, N = P.n_points, F = P.F;
+    const int p0 = blockIdx.y * W.ppb, p1 = min(N, p0 + W.ppb);
+    const double cl = W.misc[X_CL], cls = W.misc[X_CLS];
+    double nx = 0, ny = 0, nz = 0, q[K];
+    if (f < F) {
+        nx = P.fac[(size_t)f * 4];
+        ny = P.fac[(size_t)f * 4 + 1];
+        nz = P.fac[(size_t)f * 4 + 2];
+    }
+#pragma unroll
+    for (int d = 0; d < K; d++) q[d] = 0;
+    for (int b = p0; b < p1; b += kPtStage) {
+        const int np = min(kPtStage, p1 - b), npu = (np + kU - 1) / kU * kU;
+        __syncthreads();
+        for (int i = threadIdx.x; i < npu * (6 + K); i += kFcThreads) {
+            const int c = i / npu, j = i - c * npu;
+            const double* src = c < 6 ? W.e6 + (size_t)c * N : W.ls + (size_t)(c - 6) * N;
+            sp[c][j] = j < np ? src[b + j] : 0.0;
+        }
+        __syncthreads();
+        for (int i = 0; i < npu; i += kU) {
+            double mu[kU], mu0[kU];
+            bool vis[kU], some = false;
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                mu[u] = fma(sp[2][i + u], nz, fma(sp[1][i + u], ny, sp[0][i + u] * nx));
+                mu0[u] = fma(sp[5][i + u], nz, fma(sp[4][i + u], ny, sp[3][i + u] * nx));
+                vis[u] = mu[u] > kTinyD && mu0[u] > kTinyD;
+                some = some || vis[u];
+            }
+            if (!__any_sync(0xffffffffu, some)) continue;
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const double r = recip(vis[u] ? mu[u] + mu0[u] : 1.0);
+                const double s = vis[u] ? mu[u] * mu0[u] * fma(cls, r, cl) : 0.0;
+#pragma unroll
+                for (int d = 0; d < K; d++) q[d] = fma(sp[6 + d][i + u], s, q[d]);
+            }
+        }
+    }
+    if (f >= F) return;
+#pragma unroll
+    for (int d = 0; d < K; d++) W.q[((size_t)d * W.npb + blockIdx.y) * F + f] = q[d];
+}
+
+// A block of facets: Q_f = Area_f (sum of q over the point blocks + the
+// convexity rows' n_f . u), then its share of sum_f Q_f Dsph_fk, thread per
+// coefficient.
+template <int K>
+__global__ void __launch_bounds__(128) adj_cols(const DevProblem* __restrict__ Pp, AdjWork W) {
+    const DevProblem& P = *Pp;
+    __shared__ double sq[K][kColFacets];
+    const int f0 = blockIdx.x * kColFacets, F = P.F, C = P.C, nf = min(kColFacets, F - f0), tid = threadIdx.x;
+    for (int i = tid; i < K * kColFacets; i += 128) {
+        const int d = i / kColFacets, ff = i - d * kColFacets, f = f0 + ff;
+        double s = 0;
+        if (ff < nf) {
+            for (int b = 0; b < W.npb; b++) s += W.q[((size_t)d * W.npb + b) * F + f];
+            for (int c = 0; c < 3; c++) s = fma(P.fac[(size_t)f * 4 + c], W.misc[X_UC + 3 * d + c], s);
+            s *= W.area[f];
+        }
+        sq[d][ff] = s;
     }
     __syncthreads();
-    if (f >= P.F) return;
-    const double cl = W.misc[X_CL], cls = W.misc[X_CLS];
-    const double nx = P.fac[(size_t)f * 4 + 0], ny = P.fac[(size_t)f * 4 + 1], nz = P.fac[(size_t)f * 4 + 2];
-    double q = 0, q0 = 0;
-    for (int i = 0; i < np; i++) {
-        const double mu = sp[0][i] * nx + sp[1][i] * ny + sp[2][i] * nz;
-        const double mu0 = sp[3][i] * nx + sp[4][i] * ny + sp[5][i] * nz;
-        if (mu > kTinyD && mu0 > kTinyD) {
-            const double r = 1.0 / (mu + mu0);
-            const double s = mu * mu0 * fma(cls, r, cl);
-            q = fma(sp[6][i], s, q);
-            q0 = fma(sp[7][i], s, q0);
-        }
+    if (tid >= C) return;
+    double s[K];
+#pragma unroll
+    for (int d = 0; d < K; d++) s[d] = 0;
+#pragma unroll 4
+    for (int ff = 0; ff < nf; ff++) {
+        const double b = P.dsph[(size_t)(f0 + ff) * P.NCB + tid];
+#pragma unroll
+        for (int d = 0; d < K; d++) s[d] = fma(sq[d][ff], b, s[d]);
     }
-    W.q[(size_t)blockIdx.y * P.F + f] = q;
-    W.q0[(size_t)blockIdx.y * P.F + f] = q0;
+#pragma unroll
+    for (int d = 0; d < K; d++) W.cols[((size_t)d * W.ncol + blockIdx.x) * C + tid] = s[d];
 }
 
-// Q_f = Area_f sum over the point blocks of q (q0); thread per facet.
-__global__ void adj_qs(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= P.F) return;
-    double s = 0, s0 = 0;
-    for (int b = 0; b < W.npb; b++) {
-        s += W.q[(size_t)b * P.F + f];
-        s0 += W.q0[(size_t)b * P.F + f];
-    }
-    W.qs[f] = s * W.area[f];
-    W.qs0[f] = s0 * W.area[f];
-}
-
-// One CTA per output column k < C + 8: out_k = sum_f Q_f Dsph_fk (Q0 for the
-// first coefficient) + the convexity rows, out_{C+j} = sum_p l_p J_p,C+j;
-// block C + 8 sums the per-CTA chi2 shares in block order.
-__global__ void adj_cols(const DevProblem* __restrict__ Pp, AdjWork W) {
+// One CTA per free parameter and direction: a shape column's shares in block
+// order, or sum_p l_p J_p for a non-shape column; the first shape column is
+// J_p = y_p over the points plus the convexity rows' facet sum.  The last CTA
+// of direction 0 sums chi2.
+template <int K>
+__global__ void __launch_bounds__(256) adj_out(const DevProblem* __restrict__ Pp, AdjWork W, int items) {
     const DevProblem& P = *Pp;
     __shared__ double red[32];
-    const int k = blockIdx.x, C = P.C, F = P.F;
+    const int i = blockIdx.x, d = blockIdx.y, C = P.C, N = P.n_points, tid = threadIdx.x;
     double s = 0;
-    if (k < C) {
-        const double* q = k == 0 ? W.qs0 : W.qs;
-        for (int f = threadIdx.x; f < F; f += blockDim.x) s = fma(q[f], P.dsph[(size_t)f * P.NCB + k], s);
-    } else if (k < C + 8) {
-        const double* col = W.jns + (size_t)(k - C) * P.n_points;
-        for (int p = threadIdx.x; p < P.n_points; p += blockDim.x) s = fma(W.lam[p], col[p], s);
+    if (i == P.mfit) {
+        if (d > 0) return;
+        for (int b = tid; b < items; b += blockDim.x) s += W.x2part[b];
+        s = block_sum(s, red);
+        if (tid == 0) *W.chi2 = s;
+        return;
+    }
+    const int k = P.free_idx[i];
+    if (k > 0 && k < C) {
+        for (int b = tid; b < W.ncol; b += blockDim.x) s += W.cols[((size_t)d * W.ncol + b) * C + k];
     } else {
-        for (int b = threadIdx.x; b < W.nrb; b += blockDim.x) s += W.x2part[b];
+        const double* col = W.jns + (size_t)(k == 0 ? 8 : k - C) * N;
+        const double* lam = W.lam + (size_t)d * N;
+        for (int p = tid; p < N; p += blockDim.x) s = fma(lam[p], col[p], s);
+        if (k == 0 && tid < 3) s = fma(W.misc[X_CHK + tid], W.misc[X_UC + 3 * d + tid], s);
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) {
-        if (k < C) {
-            for (int nc = 0; nc < 3; nc++) s = fma(W.dres[nc * C + k], W.u[P.n_points + nc], s);
-            W.full[k] = s;
-        } else if (k < C + 8) {
-            W.full[k] = s;
-        } else {
-            *W.chi2 = s;
-        }
-    }
+    if (tid == 0) W.out[(size_t)d * P.mfit + i] = s;
 }
 
-// The free parameters' entries.
-__global__ void adj_out(const DevProblem* __restrict__ Pp, AdjWork W) {
-    const DevProblem& P = *Pp;
-    for (int i = threadIdx.x; i < P.mfit; i += blockDim.x) W.out[i] = W.full[P.free_idx[i]];
+template <int K>
+size_t carve(const DevProblem& P, double* base, AdjWork& W) {
+    const size_t N = P.n_points, F = P.F;
+    W.nfs = facet_slices(P);
+    W.ppb = points_per_block(P);
+    W.npb = cdiv(P.n_points, W.ppb);
+    W.ncurv = cdiv(P.F, kCurvFacets);
+    W.ncol = cdiv(P.F, kColFacets);
+    size_t o = 0;
+    auto take = [&](size_t n) {
+        double* r = base + o;
+        o += (n + 1) & ~(size_t)1;
+        return r;
+    };
+    W.misc = take(X_N);  // first: the host reads chck and the area sum there
+    W.dir = take(9 * K);
+    W.area = take(F);
+    W.z = take(K * F);
+    W.cpart = take((size_t)(4 + 3 * K) * W.ncurv);
+    W.e6 = take(6 * N);
+    W.pp = take((size_t)(kFixed + K) * W.nfs * N);
+    W.jns = take(9 * N);
+    W.y = take(N);
+    W.scale = take(N);
+    W.jv = take(K * N);
+    W.lam = take(K * N);
+    W.ls = take(K * N);
+    W.x2part = take(P.n_arows);
+    W.q = take((size_t)K * W.npb * F);
+    W.cols = take((size_t)K * W.ncol * P.C);
+    return o;
+}
+
+template <int K>
+cudaError_t launch(const DevProblem& P, const DevProblem* dP, double* work, const AdjArgs& args, AdjMode mode,
+                   double* d_out, double* d_chi2, cudaStream_t s) {
+    AdjWork W{};
+    carve<K>(P, work, W);
+    W.out = d_out;
+    W.chi2 = d_chi2;
+    W.mode = mode;
+    adj_curv<K><<<W.ncurv, 32 * kCurvFacets, 0, s>>>(dP, W, args);
+    adj_points<K><<<dim3(cdiv(P.n_points, kPtThreads), W.nfs), kPtThreads, 0, s>>>(dP, W);
+    adj_rows<K><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);
+    adj_facets<K><<<dim3(cdiv(P.F, kFcThreads), W.npb), kFcThreads, 0, s>>>(dP, W);
+    adj_cols<K><<<W.ncol, 128, 0, s>>>(dP, W);
+    adj_out<K><<<dim3(P.mfit + 1, K), 256, 0, s>>>(dP, W, P.n_arows);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t adjoint_misc_offset(const DevProblem& P) { return (size_t)P.F * 7 + 3 * (size_t)P.C; }
-
 size_t adjoint_work_doubles(const DevProblem& P) {
-    const size_t N = P.n_points, F = P.F;
-    const size_t npb = (N + kPtBlock - 1) / kPtBlock;
-    const size_t nrb = ((size_t)P.n_rows + kRowThreads - 1) / kRowThreads;
-    return 2 * (size_t)P.ma + F * 7 + 3 * (size_t)P.C + X_N + N * (8 + 6 + 7) + P.n_rows + 4 * (size_t)P.n_lc +
-           2 * npb * F + 2 * (size_t)P.ma + 8 + nrb + (size_t)kPart * kMaxSlices * N;
+    AdjWork W{};
+    const size_t one = carve<1>(P, nullptr, W), all = carve<kAdjDirs>(P, nullptr, W);
+    return one > all ? one : all;
 }
 
-cudaError_t launch_adjoint(const DevProblem& P, const DevProblem* dP, double* work, const double* d_a,
-                           const double* d_v, double* d_out, double* d_chi2, cudaStream_t s) {
-    AdjWork W{};
-    const size_t N = P.n_points, F = P.F;
-    W.npb = (int)((N + kPtBlock - 1) / kPtBlock);
-    double* o = work;
-    auto take = [&](size_t n) {
-        double* r = o;
-        o += n;
-        return r;
-    };
-    W.a = d_a;
-    W.v = d_v;
-    W.g = take(F);
-    W.area = take(F);
-    W.z = take(F);
-    W.z0 = take(F);
-    W.qs = take(F);
-    W.qs0 = take(F);
-    take(F);
-    W.dres = take(3 * (size_t)P.C);
-    W.misc = take(X_N);
-    W.y = take(N);
-    W.scale = take(N);
-    W.jv = take(N);
-    W.jv0 = take(N);
-    W.lam = take(N);
-    W.ls = take(N);
-    W.ls0 = take(N);
-    W.jns = take(8 * N);
-    W.e6 = take(6 * N);
-    W.u = take(P.n_rows);
-    W.lcw = take(4 * (size_t)P.n_lc);
-    W.q = take((size_t)W.npb * F);
-    W.q0 = take((size_t)W.npb * F);
-    W.full = take(P.ma + 8);
-    W.nrb = (int)(((size_t)P.n_rows + kRowThreads - 1) / kRowThreads);
-    W.x2part = take((size_t)W.nrb);
-    W.nfs = facet_slices(P);
-    W.pp = take((size_t)kPart * W.nfs * N);
-    W.out = d_out;
-    W.chi2 = d_chi2;
-    const int nlc = P.n_lc - 1;
-    const unsigned fb = (unsigned)((F + 255) / 256);
-    adj_curv<<<fb, 256, 0, s>>>(dP, W);
-    adj_conv<<<(unsigned)((4 + 3 * P.C + 7) / 8), 256, 0, s>>>(dP, W);
-    adj_points<<<dim3((unsigned)((N + kPtThreads - 1) / kPtThreads), (unsigned)W.nfs), kPtThreads, 0, s>>>(dP, W);
-    adj_points_fin<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(dP, W);
-    if (nlc > 0) adj_lc<<<(unsigned)nlc, 256, 0, s>>>(dP, W);
-    adj_rowsum<<<(unsigned)W.nrb, kRowThreads, 0, s>>>(dP, W);
-    if (nlc > 0) adj_lck<<<(unsigned)nlc, 256, 0, s>>>(dP, W);
-    adj_weights<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(dP, W);
-    adj_facets<<<dim3((unsigned)((F + kFcThreads - 1) / kFcThreads), (unsigned)W.npb), kFcThreads, 0, s>>>(dP, W);
-    adj_qs<<<fb, 256, 0, s>>>(dP, W);
-    adj_cols<<<(unsigned)(P.C + 9), 256, 0, s>>>(dP, W);
-    adj_out<<<1, 128, 0, s>>>(dP, W);
-    return cudaGetLastError();
+cudaError_t launch_adjoint(const DevProblem& P, const DevProblem* dP, double* work, const AdjArgs& args, AdjMode mode,
+                           double* d_out, double* d_chi2, cudaStream_t s) {
+    if (mode == kAdjUnits) return launch<kAdjDirs>(P, dP, work, args, mode, d_out, d_chi2, s);
+    return launch<1>(P, dP, work, args, mode, d_out, d_chi2, s);
 }
 
 }  // namespace psb

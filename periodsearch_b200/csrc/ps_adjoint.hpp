@@ -1,4 +1,4 @@
-// Matrix-free chi2 gradient and Gauss-Newton product (ps_adjoint.cu).
+// Matrix-free chi2 gradient and Gauss-Newton products (ps_adjoint.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,40 +8,32 @@
 
 namespace psb {
 
-// Device work arrays of one matrix-free evaluation (all carved from one
-// buffer of adjoint_work_doubles(P) doubles).
-struct AdjWork {
-    const double* a;  // [ma] parameters
-    const double* v;  // [ma] direction (zero on fixed parameters); null: gradient mode
-    double *g, *area, *z, *z0, *qs, *qs0;  // [F]
-    double* dres;                          // [3][C] convexity-row derivatives
-    double* misc;                          // scalars (blmatrix, scattering, phase, chck, conv J v)
-    double *y, *scale, *jv, *jv0, *lam, *ls, *ls0;  // [N] per point
-    double* jns;                           // [8][N] non-shape columns of J
-    double* e6;                            // [6][N] e, e0 of every point
-    double* u;                             // [n_rows] W (y_obs - y') or W J' v
-    double* lcw;                           // [4][n_lc] per-lightcurve sums
-    double *q, *q0;                        // [npb][F] per point block
-    double* full;                          // [ma + 8] result over all parameters
-    double* out;                           // [mfit] result over the free parameters
-    double* chi2;                          // [1]
-    double* x2part;                        // [nrb] chi2 per row block
-    double* pp;                            // [11][nfs][N] per-slice partial sums of the point pass
-    int npb, nrb, nfs;
+constexpr int kAdjMaxMa = 96;  // parameters at most (88 shape coefficients + 8)
+constexpr int kAdjDirs = 8;    // directions of one batched product
+
+// What a call brings along, passed to the first kernel by value.
+struct AdjArgs {
+    double a[kAdjMaxMa];  // parameters
+    double v[kAdjMaxMa];  // one direction over all parameters (zero on fixed ones)
+    int unit[kAdjDirs];   // batched: direction d is this parameter's unit vector (-1: zero)
+};
+
+enum AdjMode {
+    kAdjGradient,  // beta = J^T W (y_obs - y)
+    kAdjProduct,   // J^T W (J v)
+    kAdjUnits      // J^T W (J e) for kAdjDirs unit vectors e
 };
 
 size_t adjoint_work_doubles(const DevProblem& P);
-// Scalars of the last evaluation at work + adjoint_misc_offset(P): the
-// convexity residuals chck (3) at kAdjMiscChk, the facet-area sum at
-// kAdjMiscSarea.
-size_t adjoint_misc_offset(const DevProblem& P);
+// Scalars of the last evaluation at work: the convexity residuals chck (3) at
+// kAdjMiscChk, the facet-area sum after them.
 constexpr int kAdjMiscChk = 33;
 constexpr int kAdjMiscSarea = 36;
 // Kernel launches of one launch_adjoint call.
-constexpr int kAdjointLaunches = 12;
-// chi2 into d_chi2; d_v == nullptr: beta = J^T W (y_obs - y) into d_out,
-// else J^T W (J v) (v over all ma parameters, zero on the fixed ones).
-cudaError_t launch_adjoint(const DevProblem& P, const DevProblem* dP, double* work, const double* d_a,
-                           const double* d_v, double* d_out, double* d_chi2, cudaStream_t s);
+constexpr int kAdjointLaunches = 6;
+// chi2 into d_chi2; the result over the free parameters into d_out (mfit
+// values, kAdjDirs times mfit for kAdjUnits).
+cudaError_t launch_adjoint(const DevProblem& P, const DevProblem* dP, double* work, const AdjArgs& args, AdjMode mode,
+                           double* d_out, double* d_chi2, cudaStream_t s);
 
 }  // namespace psb

@@ -297,6 +297,17 @@ int upload_static(ps_ctx* c) {
         if (p.ia[i]) c->free_idx.push_back(i);
     std::vector<int> ints(lc);
     ints.insert(ints.end(), c->free_idx.begin(), c->free_idx.end());
+    // matrix-free form: antipodal facet pairs and the row items
+    const size_t pair_at = ints.size();
+    ints.insert(ints.end(), p.pairs->begin(), p.pairs->end());
+    ints.resize((ints.size() + 3) & ~(size_t)3);  // items are read as int4
+    const size_t row_at = ints.size();
+    for (int i = 0; i < L; i++) {
+        const int block = p.lc_rel[i] ? p.lc_points[i] : psb::kAdjRowBlock;
+        for (int r = lc_start[i]; r < lc_start[i + 1]; r += block)
+            ints.insert(ints.end(), {r, std::min(r + block, lc_start[i + 1]), p.lc_rel[i], p.lc_points[i]});
+    }
+    ints.insert(ints.end(), {N, N + 3, 0, 3});
     PSB_CUDA(c->d_lc.upload(ints, s));
     PSB_CUDA(c->d_queue.ensure(1));
 
@@ -326,6 +337,9 @@ int upload_static(ps_ctx* c) {
     d.lc_rel = c->d_lc.p + (L + 2);
     d.lc_npts = c->d_lc.p + (L + 2) + (L + 1);
     d.free_idx = c->d_lc.p + lc.size();
+    d.apair = p.pairs->empty() ? nullptr : c->d_lc.p + pair_at;
+    d.arows = c->d_lc.p + row_at;
+    d.n_arows = (int)((ints.size() - row_at) / 4);
     d.fac = c->d_fac.p;
     d.fac32 = c->d_fac32.p;
     d.dsph = c->d_dsph.p;
@@ -927,35 +941,37 @@ int ps_mrqcof(ps_ctx* c, const double* a, double* alpha, double* beta, double* c
     return PS_OK;
 }
 
+// What every matrix-free call needs: a device, rows, the facet pairs.
+static int check_adjoint(ps_ctx* c) {
+    int rc = check_ready(c, true);
+    if (rc) return rc;
+    if (!c->dp.apair) return fail(PS_ERR_LIMIT, "the facet grid has no antipodal pairs");
+    return PS_OK;
+}
+
 // Matrix-free chi2 / beta (v == nullptr) or Gauss-Newton product (v over
 // the mfit free parameters) at parameters a.
 static int run_adjoint(ps_ctx* c, const double* a, const double* v, double* chi2, double* out) {
-    int rc = check_ready(c, true);
+    int rc = check_adjoint(c);
     if (rc) return rc;
     if (!a) return fail(PS_ERR_ARG, "null parameter vector");
     PSB_CUDA(cudaSetDevice(c->device));
     const psb::DevProblem& d = c->dp;
     const size_t work = psb::adjoint_work_doubles(d);
-    PSB_CUDA(c->d_adj.ensure(work + 2 * (size_t)d.ma + d.mfit + 2));
-    double* d_work = c->d_adj.p;
-    double* d_a = d_work + work;
-    double* d_v = d_a + d.ma;
-    double* d_out = d_v + d.ma;
-    double* d_chi2 = d_out + d.mfit;
-    PSB_CUDA(cudaMemcpyAsync(d_a, a, d.ma * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    if (v) {
-        std::vector<double> vf(d.ma, 0.0);
-        for (int i = 0; i < d.mfit; i++) vf[c->free_idx[i]] = v[i];
-        PSB_CUDA(cudaMemcpyAsync(d_v, vf.data(), d.ma * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-        PSB_CUDA(cudaStreamSynchronize(c->stream));  // vf leaves scope
-    }
-    PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, d_work, d_a, v ? d_v : nullptr, d_out, d_chi2, c->stream));
+    PSB_CUDA(c->d_adj.ensure(work + d.mfit + 1));
+    double* d_out = c->d_adj.p + work;
+    psb::AdjArgs args{};
+    std::memcpy(args.a, a, d.ma * sizeof(double));
+    if (v)
+        for (int i = 0; i < d.mfit; i++) args.v[c->free_idx[i]] = v[i];
+    PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, c->d_adj.p, args, v ? psb::kAdjProduct : psb::kAdjGradient, d_out,
+                                 d_out + d.mfit, c->stream));
     for (int k = 0; k < psb::kAdjointLaunches; k++) psb::count_launch();
-    double x2 = 0;
-    if (out) PSB_CUDA(cudaMemcpyAsync(out, d_out, d.mfit * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PSB_CUDA(cudaMemcpyAsync(&x2, d_chi2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    double host[psb::kAdjMaxMa + 1];  // the result, then chi2
+    PSB_CUDA(cudaMemcpyAsync(host, d_out, (d.mfit + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     PSB_CUDA(cudaStreamSynchronize(c->stream));
-    if (chi2) *chi2 = x2;
+    if (out) std::memcpy(out, host, d.mfit * sizeof(double));
+    if (chi2) *chi2 = host[d.mfit];
     return PS_OK;
 }
 
@@ -1017,42 +1033,48 @@ int host_gauss_jordan(std::vector<double>& a, std::vector<double>& b, int n) {
     return 0;
 }
 
-// Device buffers of a Jacobian-free fit, carved from d_adj.
+// Device buffers of a Jacobian-free fit, carved from d_adj: alpha with room for
+// a whole last batch of columns, then beta, chi2 and an unused chi2.
 struct JfreeBufs {
-    double *work, *a, *units, *alpha, *beta, *chi2;
+    double *work, *alpha, *beta, *chi2;
 };
+
+size_t jfree_columns(int mfit) {
+    return (size_t)((mfit + psb::kAdjDirs - 1) / psb::kAdjDirs) * psb::kAdjDirs;
+}
 
 JfreeBufs jfree_bufs(ps_ctx* c) {
     const psb::DevProblem& d = c->dp;
     JfreeBufs B;
     B.work = c->d_adj.p;
-    B.a = B.work + psb::adjoint_work_doubles(d);
-    B.units = B.a + d.ma;
-    B.alpha = B.units + (size_t)d.mfit * d.ma;
-    B.beta = B.alpha + (size_t)d.mfit * d.mfit;
+    B.alpha = B.work + psb::adjoint_work_doubles(d);
+    B.beta = B.alpha + jfree_columns(d.mfit) * d.mfit;
     B.chi2 = B.beta + d.mfit;
     return B;
 }
 
 // One evaluation at a through the matrix-free kernels: chi2, chck, the
-// facet-area sum and, with full, beta and alpha (alpha's column k is the
-// Gauss-Newton product with the k-th free unit vector, mfit products).
+// facet-area sum and, with full, beta and alpha (alpha's columns are the
+// Gauss-Newton products with the free unit vectors, kAdjDirs at a time: the
+// pairs' geometry and scattering terms, three quarters of a product, are
+// formed once for all of them).
 int jfree_eval(ps_ctx* c, const JfreeBufs& B, const double* a, bool full, std::vector<double>& alpha,
                std::vector<double>& beta, double* scal) {
     const psb::DevProblem& d = c->dp;
-    const int mfit = d.mfit, ma = d.ma;
-    PSB_CUDA(cudaMemcpyAsync(B.a, a, ma * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, B.a, nullptr, B.beta, B.chi2, c->stream));
+    const int mfit = d.mfit;
+    psb::AdjArgs args{};
+    std::memcpy(args.a, a, d.ma * sizeof(double));
+    PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, args, psb::kAdjGradient, B.beta, B.chi2, c->stream));
     for (int k = 0; k < psb::kAdjointLaunches; k++) psb::count_launch();
-    // chck and the area sum depend on a only: read them before the products
-    const double* misc = B.work + psb::adjoint_misc_offset(d);
-    PSB_CUDA(cudaMemcpyAsync(scal + 1, misc + psb::kAdjMiscChk, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PSB_CUDA(cudaMemcpyAsync(scal + 4, misc + psb::kAdjMiscSarea, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PSB_CUDA(cudaMemcpyAsync(scal, B.chi2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    // chck and the area sum depend on a only; the products write them again
+    double host[4], x2 = 0;
+    PSB_CUDA(cudaMemcpyAsync(host, B.work + psb::kAdjMiscChk, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    PSB_CUDA(cudaMemcpyAsync(&x2, B.chi2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (full) {
-        for (int k = 0; k < mfit; k++) {
-            PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, B.a, B.units + (size_t)k * ma,
-                                         B.alpha + (size_t)k * mfit, B.chi2 + 1, c->stream));
+        for (int k = 0; k < mfit; k += psb::kAdjDirs) {
+            for (int q = 0; q < psb::kAdjDirs; q++) args.unit[q] = k + q < mfit ? c->free_idx[k + q] : -1;
+            PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, args, psb::kAdjUnits, B.alpha + (size_t)k * mfit,
+                                         B.chi2 + 1, c->stream));
             for (int q = 0; q < psb::kAdjointLaunches; q++) psb::count_launch();
         }
         std::vector<double> cols((size_t)mfit * mfit);
@@ -1072,6 +1094,8 @@ int jfree_eval(ps_ctx* c, const JfreeBufs& B, const double* a, bool full, std::v
     } else {
         PSB_CUDA(cudaStreamSynchronize(c->stream));
     }
+    scal[0] = x2;
+    for (int i = 0; i < 4; i++) scal[1 + i] = host[i];
     return PS_OK;
 }
 
@@ -1080,22 +1104,14 @@ int jfree_eval(ps_ctx* c, const JfreeBufs& B, const double* a, bool full, std::v
 extern "C" {
 
 int ps_fit_jfree(ps_ctx* c, double freq, int pole, ps_fit_result* out, double* cg_out) {
-    int rc = check_ready(c, true);
+    int rc = check_adjoint(c);
     if (rc) return rc;
     if (pole < 1 || pole > 10 || !(freq > 0) || !out) return fail(PS_ERR_ARG, "bad fit arguments");
     PSB_CUDA(cudaSetDevice(c->device));
     const psb::DevProblem& d = c->dp;
     const int ma = d.ma, mfit = d.mfit, C = d.C;
-    PSB_CUDA(c->d_adj.ensure(psb::adjoint_work_doubles(d) + (size_t)ma + (size_t)mfit * ma + (size_t)mfit * mfit +
-                             mfit + 2));
+    PSB_CUDA(c->d_adj.ensure(psb::adjoint_work_doubles(d) + jfree_columns(mfit) * mfit + mfit + 2));
     const JfreeBufs B = jfree_bufs(c);
-    {
-        std::vector<double> units((size_t)mfit * ma, 0.0);
-        for (int k = 0; k < mfit; k++) units[(size_t)k * ma + c->free_idx[k]] = 1.0;
-        PSB_CUDA(cudaMemcpyAsync(B.units, units.data(), units.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                 c->stream));
-        PSB_CUDA(cudaStreamSynchronize(c->stream));
-    }
     std::vector<double> cg(ma), atry(ma), alpha, beta, covar, da;
     psb::initial_parameters(c->prob, freq, pole, cg.data());
     double scal[5];

@@ -7,6 +7,8 @@
 
 namespace psb {
 
+constexpr int kAdjRowBlock = 256;  // rows of one item of the matrix-free row list
+
 // Per-asteroid tables, all device pointers, 0-based.
 //  rows: n_points data rows (lightcurve order) followed by 3 convexity rows.
 struct DevProblem {
@@ -28,6 +30,12 @@ struct DevProblem {
     const int* free_idx; // [mfit] parameter index of each free parameter
     const double* cg_first;  // [C]
     const double* pole0;     // [10][2]: initial beta' and lambda [rad]
+    // matrix-free form: facets by antipodal pairs [F/2][2]; row items
+    // {first row, last + 1, relative, points of the lightcurve}: each relative
+    // lightcurve, blocks of the calibrated ones, the convexity rows
+    const int* apair;
+    const int* arows;
+    int n_arows;
     // tile shapes (ps_set_tiles / ps_autotune): the fast form's facets per
     // staged chunk and alpha rows per tile, and the points sorted together
     int fch, rt, sortseg;

@@ -210,6 +210,36 @@ void sphfunc(Problem& p) {
     }
 }
 
+// The facets with their antipodes (Problem::pairs), the one with z > 0 first.
+std::shared_ptr<const std::vector<int>> antipodal_pairs(const Problem& p) {
+    auto pairs = std::make_shared<std::vector<int>>();
+    const int F = p.numfac;
+    // facets by their normal rounded to 1e-5: neighbours are 1e-2 apart or more,
+    // an image is within 1e-14 of where the symmetry puts it
+    auto cell = [](double v) { return (long)std::floor(v * 1e5 + 0.5); };
+    std::map<std::tuple<long, long, long>, int> at;
+    for (int f = 0; f < F; f++) {
+        const double* n = &p.nor[(size_t)f * 3];
+        at[std::make_tuple(cell(n[0]), cell(n[1]), cell(n[2]))] = f;
+    }
+    for (int f = 0; f < F; f++) {
+        const double* n = &p.nor[(size_t)f * 3];
+        if (!(n[2] > 0)) continue;
+        int g = -1;
+        for (long i = -1; i <= 1 && g < 0; i++)
+            for (long j = -1; j <= 1 && g < 0; j++)
+                for (long k = -1; k <= 1 && g < 0; k++) {
+                    auto it = at.find(std::make_tuple(cell(-n[0]) + i, cell(-n[1]) + j, cell(-n[2]) + k));
+                    if (it != at.end()) g = it->second;
+                }
+        if (g < 0) return std::make_shared<std::vector<int>>();
+        pairs->push_back(f);
+        pairs->push_back(g);
+    }
+    if ((int)pairs->size() != F) pairs->clear();
+    return pairs;
+}
+
 // Dense LU solve of the ellipsoid fit's normal equations, the role of the
 // reference's ludcmp/lubksb (ludcmp.c:9-68, lubksb.c:3-24), written from the
 // algorithm: Crout's LU factorisation P A = L U with implicit row scaling and
@@ -534,6 +564,7 @@ std::shared_ptr<const EllfitGrid> grid_tables(Problem& p) {
         std::vector<int> ifp;
         std::vector<double> nor, darea, at, af, pleg, dsph, fc, fs;
         std::shared_ptr<const EllfitGrid> ell;
+        std::shared_ptr<const std::vector<int>> pairs;
     };
     static std::mutex mu;
     static std::map<std::tuple<int, int, int>, Tables> cache;
@@ -552,16 +583,18 @@ std::shared_ptr<const EllfitGrid> grid_tables(Problem& p) {
             p.dsph = t.dsph;
             p.fc = t.fc;
             p.fs = t.fs;
+            p.pairs = t.pairs;
             return t.ell;
         }
     }
     trifac(p.nrows, p.ifp);
     areanorm(p);
     sphfunc(p);
+    p.pairs = antipodal_pairs(p);
     auto ell = ellfit_grid(p);
     std::lock_guard<std::mutex> lock(mu);
     if (cache.size() < 16)
-        cache.emplace(key, Tables{p.ifp, p.nor, p.darea, p.at, p.af, p.pleg, p.dsph, p.fc, p.fs, ell});
+        cache.emplace(key, Tables{p.ifp, p.nor, p.darea, p.at, p.af, p.pleg, p.dsph, p.fc, p.fs, ell, p.pairs});
     return ell;
 }
 

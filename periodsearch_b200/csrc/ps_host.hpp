@@ -7,6 +7,7 @@
 // receives equals the reference's bit for bit.
 #pragma once
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -47,6 +48,9 @@ struct Problem {
     std::vector<double> pleg;                // [f][l][m], (lmax+1)^2 per facet
     std::vector<double> fc, fs;              // [f][m], mmax+1 per facet
     std::vector<double> dsph;                // [f][k], ncoef per facet
+    // the facets by antipodal pairs, [F/2][2]: the triangulated sphere
+    // (trifac.c) is invariant under n -> -n; empty if a facet had no partner
+    std::shared_ptr<const std::vector<int>> pairs;
     std::vector<double> cg_first;            // ncoef
     std::vector<int> ia;                     // ma free/fixed flags
     double freq_start = 0, freq_end = 0, freq_step = 0;
