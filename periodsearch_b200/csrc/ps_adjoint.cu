@@ -42,14 +42,15 @@ using namespace fitcommon;
 constexpr int kCurvFacets = 8;    // adj_curv: facets per CTA (a warp each)
 constexpr int kPtThreads = 128;   // adj_points: points per CTA
 constexpr int kPairChunk = 64;    // adj_points: facet pairs staged at a time
-constexpr int kRowThreads = kAdjRowBlock;  // adj_rows
+constexpr int kRowThreads = 256;  // adj_rows
 constexpr int kFcThreads = 128;   // adj_facets: facets per CTA
 constexpr int kPtStage = 64;      // adj_facets: points staged at a time
 constexpr int kColFacets = 32;    // adj_cols: facets per CTA
+constexpr int kOutThreads = 1024; // adj_out: the non-shape columns run over all points
 constexpr int kFixed = 9;         // adj_points: sums besides the directions'
 constexpr int kMaxSlices = 32;    // adj_points: facet slices at most
 constexpr int kMaxPointBlocks = 64;  // adj_facets: point blocks at most
-constexpr int kFill = 4 * 148;    // CTAs that fill the GPU
+constexpr int kFill = 8 * 148;    // CTAs that fill the GPU
 
 // misc slots (X_CHK and X_SAREA are read by the host: kAdjMiscChk, kAdjMiscSarea)
 enum { X_B = 0, X_D = 9, X_CL = 27, X_CLS = 28, X_OMG = 29, X_P1 = 30, X_P2 = 31, X_P3 = 32, X_CHK = kAdjMiscChk,
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
 template <int K>
 __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
-    __shared__ double red[32];
+    __shared__ double red[32], sums[kFixed + K][kAdjRowBlock];
     const int tid = threadIdx.x, N = P.n_points;
     const int4 item = reinterpret_cast<const int4*>(P.arows)[blockIdx.x];  // first row, last + 1, relative, points of the curve
     double* x = W.misc;
@@ -341,16 +342,26 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
     double sy = 0, sj[K];
 #pragma unroll
     for (int d = 0; d < K; d++) sj[d] = 0;
-    for (int p = item.x + tid; p < item.y; p += kRowThreads) {
+    for (int p0 = item.x; p0 < item.y; p0 += kAdjRowBlock) {
+        // the slices' sums, in slice order, kRowThreads / kAdjRowBlock threads per point
+        const int np = min(kAdjRowBlock, item.y - p0), i0 = tid % kAdjRowBlock;
+        __syncthreads();
+        if (i0 < np)
+            for (int j = tid / kAdjRowBlock; j < kFixed + K; j += kRowThreads / kAdjRowBlock) {
+                const double* src = W.pp + (size_t)j * W.nfs * N + p0 + i0;
+                double v = 0;
+#pragma unroll 8
+                for (int k = 0; k < W.nfs; k++) v += src[(size_t)k * N];
+                sums[j][i0] = v;
+            }
+        __syncthreads();
+        if (tid >= np) continue;
+        const int p = p0 + tid;
         PointGeom G;
         point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
         double acc[kFixed + K];
 #pragma unroll
-        for (int j = 0; j < kFixed + K; j++) {
-            double v = 0;
-            for (int k = 0; k < W.nfs; k++) v += W.pp[((size_t)j * W.nfs + k) * N + p];
-            acc[j] = v;
-        }
+        for (int j = 0; j < kFixed + K; j++) acc[j] = sums[j][tid];
         const double br = acc[0], sc = G.scale, yy = br * sc;
         double jn[9];
         for (int k = 0; k < 3; k++) {
@@ -509,7 +520,7 @@ __global__ void __launch_bounds__(128) adj_cols(const DevProblem* __restrict__ P
 // J_p = y_p over the points plus the convexity rows' facet sum.  The last CTA
 // of direction 0 sums chi2.
 template <int K>
-__global__ void __launch_bounds__(256) adj_out(const DevProblem* __restrict__ Pp, AdjWork W, int items) {
+__global__ void __launch_bounds__(kOutThreads) adj_out(const DevProblem* __restrict__ Pp, AdjWork W, int items) {
     const DevProblem& P = *Pp;
     __shared__ double red[32];
     const int i = blockIdx.x, d = blockIdx.y, C = P.C, N = P.n_points, tid = threadIdx.x;
@@ -527,7 +538,8 @@ __global__ void __launch_bounds__(256) adj_out(const DevProblem* __restrict__ Pp
     } else {
         const double* col = W.jns + (size_t)(k == 0 ? 8 : k - C) * N;
         const double* lam = W.lam + (size_t)d * N;
-        for (int p = tid; p < N; p += blockDim.x) s = fma(lam[p], col[p], s);
+#pragma unroll 4
+        for (int p = tid; p < N; p += kOutThreads) s = fma(__ldg(lam + p), __ldg(col + p), s);
         if (k == 0 && tid < 3) s = fma(W.misc[X_CHK + tid], W.misc[X_UC + 3 * d + tid], s);
     }
     s = block_sum(s, red);
@@ -580,7 +592,7 @@ cudaError_t launch(const DevProblem& P, const DevProblem* dP, double* work, cons
     adj_rows<K><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);
     adj_facets<K><<<dim3(cdiv(P.F, kFcThreads), W.npb), kFcThreads, 0, s>>>(dP, W);
     adj_cols<K><<<W.ncol, 128, 0, s>>>(dP, W);
-    adj_out<K><<<dim3(P.mfit + 1, K), 256, 0, s>>>(dP, W, P.n_arows);
+    adj_out<K><<<dim3(P.mfit + 1, K), kOutThreads, 0, s>>>(dP, W, P.n_arows);
     return cudaGetLastError();
 }
 

@@ -7,7 +7,7 @@
 
 namespace psb {
 
-constexpr int kAdjRowBlock = 256;  // rows of one item of the matrix-free row list
+constexpr int kAdjRowBlock = 64;  // rows of one item of the matrix-free row list
 
 // Per-asteroid tables, all device pointers, 0-based.
 //  rows: n_points data rows (lightcurve order) followed by 3 convexity rows.

@@ -573,6 +573,7 @@ __device__ __forceinline__ void alpha_tensor(const DevProblem& P, const double* 
         }
         const double* jb = work + b * bstride;
         const double* wb = jb + rt * st;
+#pragma unroll 4
         for (int rr = 0; rr < nr4; rr += 4) {
             const double* row = jb + (rr + q) * st + g;
             const double w = wb[rr + q];
