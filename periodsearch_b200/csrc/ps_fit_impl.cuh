@@ -635,9 +635,12 @@ __device__ __forceinline__ void eval_scalars(const double* a, int C, double* B, 
 
 // curv.c:15-37: g = exp(sum over (m, l) of Pleg * (c*Fc + s*Fs)), thread per
 // facet; area = Darea g, zero for the 128 slots past F.
-__device__ __forceinline__ void curv_phase(const DevProblem& P, const double* a, double* g, double* area,
+// Returns whether this thread's g are all of ordinary size (g Dsph cannot
+// overflow).
+__device__ __forceinline__ bool curv_phase(const DevProblem& P, const double* a, double* g, double* area,
                                            bool pad = true) {
     const int F = P.F;
+    bool ordinary = true;
     for (int f = threadIdx.x; f < F; f += kThreads) {
         const double* pl = P.cpl + (size_t)f * P.nq;
         const double* fc = P.cfc + (size_t)f * (P.mmax + 1);
@@ -658,11 +661,13 @@ __device__ __forceinline__ void curv_phase(const DevProblem& P, const double* a,
             }
         }
         gi = exp(gi);
+        ordinary = ordinary && gi < 1e200;
         g[f] = gi;
         area[f] = P.fac[(size_t)f * 4 + 3] * gi;
     }
     if (pad)
         for (int f = F + threadIdx.x; f < F + 128; f += kThreads) area[f] = 0.0;
+    return ordinary;
 }
 
 // chi2 over all rows (mrqcof.c:119-135) from the normalised model yt.  The
@@ -919,13 +924,17 @@ __device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, i
 // points, 800 facets and 49 coefficients: 314 ms with one facet at a time, three
 // or four IEEE divisions each, inlined; 277 with two facets and one reciprocal;
 // 261 out of line; 253 with the halves balanced (ref_halves; one facet: 286,
-// four: 276, which need more than 128 registers).  With few coefficients four
-// fit: 500 points and 16 coefficients, 140 fits and 400: 112 -> 109 ms.
+// four: 276, which need more than 128 registers).  With few coefficients
+// (kFlat) registers are left to run the sums' products side by side too, and
+// the pass is a chain of latencies: one fit of 118 points and 16 coefficients
+// 6.3 -> 5.8 ms, the pre-pass and 400 fits of 500 points 104 -> 97 ms; 290 fits
+// of 500 points and 25 coefficients 34.3 -> 32.3, of 700 and 36 60 -> 58; at 49
+// coefficients 249 -> 256.
 // `p`: the thread's point, -1 for none.  first: also the facet sums.  want_cl, all: also the columns of the
 // Lambert coefficient, of the (never fitted) Lommel-Seeliger one.
 template <int NCB, int H, int kFirst, int kCount>
-__device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool first, bool want_cl, bool all,
-                                      double* Jt, double* yt) {
+__device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool first, bool ordinary,
+                                      bool want_cl, bool all, double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const DevProblem& P = *Pp;
     const Layout L = make_layout(P);
@@ -940,7 +949,8 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
     const int pl = threadIdx.x & (kThreads / 2 - 1);
     const bool act = p >= 0;
     constexpr int kPts = kThreads / 2;
-    constexpr int kU = NCB <= 24 ? 4 : 2;  // facets at a time
+    constexpr int kU = 2;              // facets at a time
+    constexpr bool kFlat = NCB <= 40;  // the sums without a branch too
     const int tid = threadIdx.x;
     const int F = P.F, C = P.C, npad = P.npad;
     const double cl = misc[M_CL], cls = misc[M_CLS];
@@ -1039,6 +1049,42 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
                 cmu[u] = mu;
                 cmu0[u] = mu0;
             }
+            if (kFlat && ordinary) {
+                // a facet the lane does not see adds zeros, which leave the sums as
+                // they are as long as g Dsph is finite
+                double t0[kU], t1[kU], t2[kU], dbr[kU];
+#pragma unroll
+                for (int u = 0; u < kU; u++) {
+                    const double* fp = fq + 5 * u;
+                    const double nx = fp[0], ny = fp[1], nz = fp[2], ar = fp[3];
+                    dbr[u] = vis[u] ? fp[4] * sv[u] : 0.0;
+                    const double sum = nx * dv[0] + ny * dv[kPts] + nz * dv[2 * kPts];
+                    const double sum0 = nx * dv[3 * kPts] + ny * dv[4 * kPts] + nz * dv[5 * kPts];
+                    t1[u] = vis[u] ? ar * (dsmu[u] * sum + dsmu0[u] * sum0) : 0.0;
+                    if constexpr (H == 0) {
+                        t0[u] = vis[u] ? ar * sv[u] : 0.0;
+                        const double s2 = nx * dv[6 * kPts] + ny * dv[7 * kPts] + nz * dv[8 * kPts];
+                        const double s20 = nx * dv[9 * kPts] + ny * dv[10 * kPts] + nz * dv[11 * kPts];
+                        t2[u] = vis[u] ? ar * (dsmu[u] * s2 + dsmu0[u] * s20) : 0.0;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kU; u++) {
+                    const double* dg = s_dg + (f1 + u) * NCB + kFirst;
+#pragma unroll
+                    for (int k = 0; k < kCount; k++) acc[k] = acc[k] + dbr[u] * dg[k];
+                    a1 = a1 + t1[u];
+                    if constexpr (H == 0) {
+                        a0 = a0 + t0[u];
+                        a2 = a2 + t2[u];
+                    } else if (want_cl && vis[u]) {
+                        const double ar = fq[5 * u + 3];
+                        a0 = a0 + cmu[u] * cmu0[u] * ar;
+                        if (all) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
+                    }
+                }
+                continue;
+            }
 #pragma unroll
             for (int u = 0; u < kU; u++) {
                 if (!vis[u]) continue;
@@ -1102,19 +1148,19 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
 // derivative and brightness sum are 17 operations per pair, the shape sums 2
 // each, so half 1 takes eight more of them.
 template <int NCB, int kTotal>
-__device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool first, bool want_cl,
-                                           bool all, double* Jt, double* yt) {
+__device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool first, bool ordinary,
+                                           bool want_cl, bool all, double* Jt, double* yt) {
     constexpr int k0 = kTotal > 9 ? (kTotal - 8) / 2 & ~1 : 0;  // even: dg is read in pairs
     if (h == 0)
-        ref_pass<NCB, 0, 0, k0>(Pp, p, first, want_cl, all, Jt, yt);
+        ref_pass<NCB, 0, 0, k0>(Pp, p, first, ordinary, want_cl, all, Jt, yt);
     else
-        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, first, want_cl, all, Jt, yt);
+        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, first, ordinary, want_cl, all, Jt, yt);
 }
 
 // ref_pass over every data point, in segments sorted by viewing direction.
 template <int NCB>
-__device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp, double* sm, const Layout& L, bool all,
-                                               double* Jt, double* yt) {
+__device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp, double* sm, const Layout& L,
+                                               bool ordinary, bool all, double* Jt, double* yt) {
     constexpr int kPts = kThreads / 2;
     const DevProblem& P = *Pp;
     const int tid = threadIdx.x, h = tid / kPts, pl = tid - h * kPts;
@@ -1132,9 +1178,9 @@ __device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp
             const bool first = s0 == 0 && base == 0;
             // C = 1 mod 8 for every even lmax = mmax: no sums for the padding
             if (P.C > NCB - 7)
-                ref_halves<NCB, NCB>(Pp, h, p, first, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB>(Pp, h, p, first, ordinary, want_cl, all, Jt, yt);
             else
-                ref_halves<NCB, NCB - 7>(Pp, h, p, first, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB - 7>(Pp, h, p, first, ordinary, want_cl, all, Jt, yt);
         }
     }
 }
@@ -1255,8 +1301,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
     double* work = sm + L.work;
 
     eval_scalars(a, C, B, D, misc);
-    curv_phase(P, a, g, area);
-    __syncthreads();
+    const bool ordinary = __syncthreads_and(curv_phase(P, a, g, area));
     if constexpr (kFast) {
         if constexpr (NCB >= 16) {
             if (C == NCB - 7)
@@ -1267,7 +1312,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
             point_loop_fast<NCB, false>(Pp, Jt, yt);
         }
     } else {
-        point_loop_ref<NCB>(Pp, sm, L, all, Jt, yt);
+        point_loop_ref<NCB>(Pp, sm, L, ordinary, all, Jt, yt);
     }
     __syncthreads();
     // convexity rows (conv.c:12-29): y = residual, J = dres for the shape

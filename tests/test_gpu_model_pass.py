@@ -6,6 +6,7 @@ around a warp, a block of 256 threads and the four points a thread takes."""
 import numpy as np
 import pytest
 
+from conftest import golden_path
 from periodsearch_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -60,4 +61,29 @@ def test_jacobian_rows_at_any_scattering(native, oracle_lib, tmp_path, form, nro
             # a column may be what cancellation leaves: its scale is J's at least
             scale = max(np.linalg.norm(J_o[:, k]), 1e-3 * np.linalg.norm(J_o) / np.sqrt(g.ma))
             assert np.linalg.norm(J[:, k] - J_o[:, k]) <= 1e-11 * scale, (log_cl, cls, k)
+    g.close()
+
+
+def test_jacobian_of_an_overflowing_shape(native, oracle_lib):
+    """Facet areas of 1e204: the reference-order form's sums then take the
+    branch that leaves facets out which a point does not see."""
+    path = golden_path("tiny")
+    o = oracle_lib.Oracle(path)
+    o.set_conw_r(o.conw_r)
+    g = native.PeriodSearch(path, form=native.PS_FORM_FP64)
+    g.set_conw_r(o.conw_r)
+    a = o.initial_parameters(o.freq(1), 2)
+    a[0] = 470.0
+    y_o, J_o = o.model(a)
+    y, J = g.model(a)
+    # the products of the relative-lightcurve normalisation overflow: the same
+    # entries must, and the others agree
+    fine = np.isfinite(J_o)
+    assert np.array_equal(fine, np.isfinite(J)) and np.abs(J_o[fine]).max() > 1e200 and np.all(np.isfinite(y_o))
+    top = np.abs(J_o[fine]).max()
+    for got, ref, ok in [(y, y_o, np.isfinite(y_o))] + [(J[:, k], J_o[:, k], fine[:, k]) for k in range(g.ma)]:
+        # an exponent of 470 carries 470 roundings of exp's argument: 1e-13; a
+        # column may be what cancellation leaves
+        if ok.any():
+            assert np.abs(got[ok] - ref[ok]).max() <= 1e-9 * max(np.abs(ref[ok]).max(), 1e-6 * top)
     g.close()
