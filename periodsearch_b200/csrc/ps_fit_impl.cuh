@@ -287,13 +287,14 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // facets -- and the warp multiplies the 8x4 A tile into the 8 x NCB accumulator
 // tiles with m8n8k4 FP64 MMAs (B = dsph rows from shared memory).  A step with
 // no visible (point, facet) pair skips its MMAs.  Out of line, for the
-// registers.  Bound by the latency of a step's chain and by instruction issue;
-// one reciprocal without a branch instead of the IEEE division's: 140 fits of
-// 20 000 points, 2048 facets and 81 coefficients 304 -> 258 ms, 2400 fits of 760
-// points, 800 facets and 49 coefficients unchanged (92 ms; there two steps go
-// side by side, which one CTA per SM does not need: 262 ms).  Facet chunks are staged with asynchronous copies, one chunk
-// ahead.  Sums split by facet (lane q takes facets q mod 4) are combined at
-// the end: the form differs from the reference order by rounding only.
+// registers.  Bound by the latency of a step's chain and by instruction issue:
+// one reciprocal without a branch instead of the IEEE division's, and normals
+// read in pairs, took 140 fits of 20 000 points, 2048 facets and 81 coefficients
+// from 304 to 254 ms and 2400 fits of 760 points, 800 facets and 49 coefficients
+// from 92.5 to 87.0 (two steps side by side: 90.7).
+// Facet chunks are staged with asynchronous copies, one chunk ahead.  Sums
+// split by facet (lane q takes facets q mod 4) are combined at the end: the form
+// differs from the reference order by rounding only.
 // kX1 (C = NCB - 7, i.e. C = 1 mod 8 as for every even lmax = mmax): the last
 // 8-column tile would carry a single coefficient, so coefficient C - 1 is
 // summed per lane on the FP64 pipe (one FMA per visible pair) and the MMA
@@ -312,7 +313,6 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
     double* work = sm + L.work;
     constexpr int NT = kX1 ? NCB / 8 - 1 : NCB / 8;  // MMA accumulator tiles per 8 points
     static_assert(NT > 0, "kX1 needs NCB >= 16");
-    constexpr int kU = NCB <= 64 ? 2 : 1;            // steps of four facets at a time
     constexpr int kPts = (kThreads / 32) * 8;        // points per pass
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, q = lane & 3;
@@ -387,57 +387,36 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
                 }
                 // Facets past F (zero rows in the staged chunk, zero area) and
                 // inactive lanes (e = e0 = 0) have mu = mu0 = 0: not visible.
-                // kU steps of four facets at a time: their per-pair terms without a
-                // branch, side by side (a facet the lane does not see counts with
-                // area 0, which leaves every sum as it is), then the MMAs.
-                for (int j = 0; j < nf; j += 4 * kU) {
-                    double mu[kU], mu0[kU], ar[kU], av[kU];
-                    bool any[kU], some = false;
+                // A step whose pairs some lane sees runs without a branch: a facet the
+                // lane does not see counts with area 0, which leaves every sum as it is.
+                for (int j = 0; j < nf; j += 4) {
+                    const int ff = j + q;
+                    const double2 nxy = *reinterpret_cast<const double2*>(fb + ff * 4);
+                    const double nz = fb[ff * 4 + 2];
+                    const double mu = fma(e[2], nz, fma(e[0], nxy.x, e[1] * nxy.y));
+                    const double mu0 = fma(e0[2], nz, fma(e0[0], nxy.x, e0[1] * nxy.y));
+                    const bool vis = (mu > kTinyD) && (mu0 > kTinyD);
+                    if (!__any_sync(full, vis)) continue;
+                    const double ar = vis ? area[f0 + ff] : 0.0;
+                    const double r = QuotientsBy(vis ? mu + mu0 : 1.0).y;
+                    const double av = ar * (mu * mu0 * fma(cls, r, cl));
+                    br = __dadd_rn(br, av);
+                    const double q0 = mu0 * r, q1 = mu * r;
+                    const double w = ar * fma(cls * q0, q0, cl * mu0);
+                    const double w0 = ar * fma(cls * q1, q1, cl * mu);
+                    T[0] = fma(w, nxy.x, T[0]);
+                    T[1] = fma(w, nxy.y, T[1]);
+                    T[2] = fma(w, nz, T[2]);
+                    S[0] = fma(w0, nxy.x, S[0]);
+                    S[1] = fma(w0, nxy.y, S[1]);
+                    S[2] = fma(w0, nz, S[2]);
+                    const double mm = mu * mu0 * ar;
+                    s_cl += mm;
+                    s_cls = fma(mm, r, s_cls);
+                    if (kX1) x1 = fma(av, db[ff * kDs<NCB> + 8 * NT], x1);
+                    const double* brow = db + ff * kDs<NCB> + g;
 #pragma unroll
-                    for (int u = 0; u < kU; u++) {
-                        const int ff = j + 4 * u + q;
-                        const bool in = kU == 1 || j + 4 * u < nf;
-                        const double* n = fb + (in ? ff : q) * 4;
-                        mu[u] = fma(e[2], n[2], fma(e[0], n[0], e[1] * n[1]));
-                        mu0[u] = fma(e0[2], n[2], fma(e0[0], n[0], e0[1] * n[1]));
-                        const bool vis = in && (mu[u] > kTinyD) && (mu0[u] > kTinyD);
-                        any[u] = __any_sync(full, vis);
-                        some = some || any[u];
-                        ar[u] = vis ? area[f0 + ff] : 0.0;
-                        av[u] = vis ? mu[u] + mu0[u] : 1.0;
-                    }
-                    if (!some) continue;
-#pragma unroll
-                    for (int u = 0; u < kU; u++) av[u] = QuotientsBy(av[u]).y;
-#pragma unroll
-                    for (int u = 0; u < kU; u++) {
-                        const int ff = j + 4 * u + q;
-                        const double* n = fb + (kU == 1 || j + 4 * u < nf ? ff : q) * 4;
-                        const double r = av[u];
-                        const double sv = mu[u] * mu0[u] * fma(cls, r, cl);
-                        av[u] = ar[u] * sv;
-                        br = __dadd_rn(br, av[u]);
-                        const double q0 = mu0[u] * r, q1 = mu[u] * r;
-                        const double w = ar[u] * fma(cls * q0, q0, cl * mu0[u]);
-                        const double w0 = ar[u] * fma(cls * q1, q1, cl * mu[u]);
-                        T[0] = fma(w, n[0], T[0]);
-                        T[1] = fma(w, n[1], T[1]);
-                        T[2] = fma(w, n[2], T[2]);
-                        S[0] = fma(w0, n[0], S[0]);
-                        S[1] = fma(w0, n[1], S[1]);
-                        S[2] = fma(w0, n[2], S[2]);
-                        const double mm = mu[u] * mu0[u] * ar[u];
-                        s_cl += mm;
-                        s_cls = fma(mm, r, s_cls);
-                        if (kX1) x1 = fma(av[u], db[(kU == 1 || j + 4 * u < nf ? ff : q) * kDs<NCB> + 8 * NT], x1);
-                    }
-#pragma unroll
-                    for (int u = 0; u < kU; u++) {
-                        if (!any[u]) continue;
-                        const double* brow = db + (j + 4 * u + q) * kDs<NCB> + g;
-#pragma unroll
-                        for (int t = 0; t < NT; t++) dmma_8x8x4(acc[t][0], acc[t][1], av[u], brow[t * 8]);
-                    }
+                    for (int t = 0; t < NT; t++) dmma_8x8x4(acc[t][0], acc[t][1], av, brow[t * 8]);
                 }
                 cp_async_wait_all();
                 __syncthreads();
