@@ -225,13 +225,12 @@ std::shared_ptr<const std::vector<int>> antipodal_pairs(const Problem& p) {
     for (int f = 0; f < F; f++) {
         const double* n = &p.nor[(size_t)f * 3];
         if (!(n[2] > 0)) continue;
-        int g = -1;
-        for (long i = -1; i <= 1 && g < 0; i++)
-            for (long j = -1; j <= 1 && g < 0; j++)
-                for (long k = -1; k <= 1 && g < 0; k++) {
-                    auto it = at.find(std::make_tuple(cell(-n[0]) + i, cell(-n[1]) + j, cell(-n[2]) + k));
-                    if (it != at.end()) g = it->second;
-                }
+        // the image's own cell, and its neighbours where rounding split the two
+        const long c[3] = {cell(-n[0]), cell(-n[1]), cell(-n[2])};
+        auto it = at.find(std::make_tuple(c[0], c[1], c[2]));
+        for (int k = 0; k < 27 && it == at.end(); k++)
+            it = at.find(std::make_tuple(c[0] + k / 9 - 1, c[1] + k / 3 % 3 - 1, c[2] + k % 3 - 1));
+        const int g = it == at.end() ? -1 : it->second;
         if (g < 0) return std::make_shared<std::vector<int>>();
         pairs->push_back(f);
         pairs->push_back(g);
