@@ -289,9 +289,9 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // no visible (point, facet) pair skips its MMAs.  Out of line, for the
 // registers.  Bound by the latency of a step's chain and by instruction issue:
 // one reciprocal without a branch instead of the IEEE division's, and normals
-// read in pairs, took 140 fits of 20 000 points, 2048 facets and 81 coefficients
-// from 304 to 254 ms and 2400 fits of 760 points, 800 facets and 49 coefficients
-// from 92.5 to 87.0 (two steps side by side: 90.7).
+// read in pairs, took 2400 fits of 760 points, 800 facets and 49 coefficients
+// from 92.5 to 87.0 ms (two steps side by side: 90.7) and 140 fits of 20 000
+// points, 2048 facets and 81 coefficients, one CTA per SM, from 305 to 302.
 // Facet chunks are staged with asynchronous copies, one chunk ahead.  Sums
 // split by facet (lane q takes facets q mod 4) are combined at the end: the form
 // differs from the reference order by rounding only.
