@@ -123,17 +123,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// 1 / d for d in (2e-8, 2], correctly rounded but for a handful of operands:
-// the hardware's approximation, a cubic and a Newton step.  No branch.
-__device__ __forceinline__ double recip(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    double e = fma(-d, r, 1.0);
-    r = fma(r, fma(e, e, e), r);
-    e = fma(-d, r, 1.0);
-    return fma(r, e, r);
-}
-
 // blmatrix, the scattering and phase scalars and the directions' non-shape
 // parts (block 0); curv (curv.c:15-37 through Dsph = Fc/Fs Pleg), z without the
 // first coefficient, and each CTA's share of the facet sums: a warp per facet,
@@ -272,7 +261,7 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
             const double mu0 = fma(e0[2], nz, fma(e0[1], ny, e0[0] * nx));
             const bool vis = mu > kTinyD && mu0 > kTinyD;
             const double ar = vis ? sf[3][i] : 0.0;
-            const double r = recip(vis ? mu + mu0 : 1.0);
+            const double r = rcp_newton(vis ? mu + mu0 : 1.0);
             const double am = ar * mu, am0 = ar * mu0, mm = am * mu0, cr = cls * r, crr = cr * r;
             const double t = mm * (cr + cl);
             acc[0] += t;                      // br
@@ -470,7 +459,7 @@ __global__ void __launch_bounds__(kFcThreads) adj_facets(const DevProblem* __res
             if (!__any_sync(0xffffffffu, some)) continue;
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                const double r = recip(vis[u] ? mu[u] + mu0[u] : 1.0);
+                const double r = rcp_newton(vis[u] ? mu[u] + mu0[u] : 1.0);
                 const double s = vis[u] ? mu[u] * mu0[u] * fma(cls, r, cl) : 0.0;
 #pragma unroll
                 for (int d = 0; d < K; d++) q[d] = fma(sp[6 + d][i + u], s, q[d]);

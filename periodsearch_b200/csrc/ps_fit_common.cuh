@@ -18,6 +18,52 @@ constexpr int kThreads = 256;
 constexpr double kPiD = 3.14159265358979323846;
 constexpr double kTinyD = 1e-8;  // constants.h:10
 
+// 1 / x for x of ordinary size (mu + mu0 of a visible pair), to rounding: the
+// hardware's approximation (2^-20) refined by two Newton-Raphson steps
+// r <- r + r (1 - x r), each of which squares the relative error.  No branch.
+__device__ __forceinline__ double rcp_newton(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    double e = fma(-x, r, 1.0);
+    r = fma(r, e, r);
+    e = fma(-x, r, 1.0);
+    return fma(r, e, r);
+}
+
+// 1 / x likewise, rounded to nearest: a third step, taken from a value within
+// an ulp, rounds correctly (P. Markstein, Computation of elementary functions on
+// the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990) unless x's
+// mantissa is all ones, where 1 / x lies just above the middle of two numbers;
+// the second step rounds up so that the third comes to it from above and is
+// right there too.
+__device__ __forceinline__ double rcp_nearest(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    double e = fma(-x, r, 1.0);
+    r = fma(r, e, r);
+    e = fma(-x, r, 1.0);
+    r = __fma_ru(r, e, r);
+    e = fma(-x, r, 1.0);
+    return fma(r, e, r);
+}
+
+// Quotients a / d of one divisor with IEEE rounding, as the reference's
+// divisions give them: y = 1 / d to nearest, q = a y, then Markstein's step
+// q + y (a - d q), which rounds correctly: it is off by less than
+// 2^-53 |a / d - q| before its rounding, and where a / d lies so close to a middle
+// that this could matter, q is one of its two neighbours.  a and d of ordinary
+// size (no overflow, underflow or special value anywhere on the way; a may be
+// zero).  No branch and no call, unlike the division, so several run side by
+// side.
+struct QuotientsBy {
+    double d, y;
+    __device__ __forceinline__ explicit QuotientsBy(double divisor) : d(divisor), y(rcp_nearest(divisor)) {}
+    __device__ __forceinline__ double of(double a) const {
+        const double q = a * y;
+        return fma(fma(-d, q, a), y, q);
+    }
+};
+
 // blmatrix.c:9-46.  B[i*3+j] = Blmat[i+1][j+1]; D[(d*3+i)*3+j] = Dblm[d+1][i+1][j+1].
 __device__ void blmatrix(double bet, double lam, double* B, double* D) {
     double cb = cos(bet), sb = sin(bet), cl = cos(lam), sl = sin(lam);

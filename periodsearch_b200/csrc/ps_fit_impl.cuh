@@ -27,44 +27,9 @@ constexpr int kMf = 128;     // facets per staged chunk of the model-only pass
 
 constexpr int kMp = 4;       // points per thread at most in the model-only pass
 
-// 1/x for x in (2e-8, 2] (mu + mu0 of a visible pair), fast form only: the
-// hardware's approximate FP64 reciprocal refined by two Newton-Raphson steps
-// r <- r + r (1 - x r), each of which squares the relative error, so the
-// result is within rounding of the IEEE quotient.
-__device__ __forceinline__ double rcp_newton(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
-    return fma(r, e, r);
-}
 // The fast form takes its facet-chunk and alpha row-tile sizes and both forms
 // the point-sort segment from the problem (DevProblem::fch, rt, sortseg):
 // runtime tile shapes, chosen by ps_autotune; no choice changes any result.
-
-// Quotients a / d of one divisor with IEEE rounding, as the reference's
-// divisions give them: y = RN(1 / d) (the hardware's approximate reciprocal, a
-// cubic and a final Newton step), then q = a y and one residual step
-// q + y (a - d q) in fused arithmetic, which rounds correctly when y does
-// (Markstein, IBM J. Res. Dev. 34, 1990).  For d in (2e-8, 4] and a of ordinary
-// magnitude (no overflow, underflow or special value anywhere on the way).
-// No branch and no call, unlike the division, so several run side by side.
-struct QuotientsBy {
-    double d, y;
-    __device__ __forceinline__ explicit QuotientsBy(double divisor) : d(divisor) {
-        double r;
-        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-        double e = fma(-d, r, 1.0);
-        r = fma(r, fma(e, e, e), r);
-        e = fma(-d, r, 1.0);
-        y = fma(r, e, r);
-    }
-    __device__ __forceinline__ double of(double a) const {
-        const double q = a * y;
-        return fma(fma(-d, q, a), y, q);
-    }
-};
 
 // Blocks of the alpha/beta/chi2 accumulation for mfit free parameters: for
 // each even j0 <= mfit - 1, the 4-column blocks k0 = 4 kb of the lower
@@ -398,7 +363,7 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
                     const bool vis = (mu > kTinyD) && (mu0 > kTinyD);
                     if (!__any_sync(full, vis)) continue;
                     const double ar = vis ? area[f0 + ff] : 0.0;
-                    const double r = QuotientsBy(vis ? mu + mu0 : 1.0).y;
+                    const double r = rcp_nearest(vis ? mu + mu0 : 1.0);
                     const double av = ar * (mu * mu0 * fma(cls, r, cl));
                     br = __dadd_rn(br, av);
                     const double q0 = mu0 * r, q1 = mu * r;
