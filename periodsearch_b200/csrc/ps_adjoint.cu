@@ -13,10 +13,11 @@
 // non-shape columns are formed per point, and so is the first shape column:
 // Dsph_f0 = 1, so it is the model itself, and z leaves the first coefficient
 // out.  The relative-lightcurve normalisation (mrqcof.c:92-104),
-// J'_r = coef (J_r - y_r dave / ave) with dave = sum_r J_r and J'_r1 = 0,
+// J'_r = coef_r (J_r - y_r dave / ave) with dave = sum_r J_r and J'_r1 = 0,
 // becomes per-lightcurve scalars:
-//   (J' v)_r  = coef ((J v)_r - y_r sum_{r'} (J v)_{r'} / ave)   (v_1 left out)
-//   J'^T u    = J^T l,  l_r = coef (u_r - sum_{r'} y_{r'} u_{r'} / ave).
+//   (J' v)_r  = coef_r ((J v)_r - y_r sum_{r'} (J v)_{r'} / ave)   (v_1 left out)
+//   J'^T u    = J^T l,  l_r = coef_r u_r - sum_{r'} coef_{r'} y_{r'} u_{r'} / ave;
+// coef_r = sigma_r L / ave: a curve's sigmas need not be equal.
 // A convexity row (conv.c:12-29) is a point whose s_pf is a component of the
 // facet's normal, so its weights join the facet sums.  Every reduction runs in
 // a fixed order, so results are deterministic.
@@ -378,7 +379,10 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
             sj[d] += s;
         }
     }
+    // coef of a row: L sigma / ave; rs is its sigma over the curve's first, one
+    // for the per-curve mean
     double ave = 0, sjv[K], kap[K], coefn = 0;
+    const double sig0 = rel ? P.sig[item.x] : 1.0;
 #pragma unroll
     for (int d = 0; d < K; d++) sjv[d] = kap[d] = 0;
     if (rel) {
@@ -388,7 +392,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         for (int d = 0; d < K; d++) sjv[d] = block_sum(sj[d], red) / ave;
     }
     for (int p = item.x + tid; p < item.y; p += kRowThreads) {
-        const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0;
+        const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0, rs = rel ? P.sig[p] / sig0 : 1.0;
         const double w = P.sig2i[p] * P.wght[p], dy = P.yobs[p] - coef * y;
         x2 = fma(dy * w, dy, x2);
 #pragma unroll
@@ -396,7 +400,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
             const double jv = W.jv[(size_t)d * N + p];
             const double u = W.mode == kAdjGradient ? w * dy : w * (rel ? coef * (jv - y * sjv[d]) : jv);
             W.lam[(size_t)d * N + p] = u;
-            kap[d] = fma(y, u, kap[d]);
+            kap[d] = fma(rs * y, u, kap[d]);
         }
     }
     if (rel) {
@@ -404,11 +408,11 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         for (int d = 0; d < K; d++) kap[d] = block_sum(kap[d], red) / ave;
     }
     for (int p = item.x + tid; p < item.y; p += kRowThreads) {
-        const double sc = W.scale[p], coef = rel ? P.sig[p] * coefn : 1.0;
+        const double sc = W.scale[p], coef0 = sig0 * coefn, rs = rel ? P.sig[p] / sig0 : 1.0;
 #pragma unroll
         for (int d = 0; d < K; d++) {
             double l = W.lam[(size_t)d * N + p];
-            if (rel) l = coef * (l - kap[d]);
+            if (rel) l = coef0 * (rs * l - kap[d]);
             W.lam[(size_t)d * N + p] = l;
             W.ls[(size_t)d * N + p] = l * sc;
         }
