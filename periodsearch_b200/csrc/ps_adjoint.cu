@@ -22,11 +22,12 @@
 // facet's normal, so its weights join the facet sums.  Every reduction runs in
 // a fixed order, so results are deterministic.
 //
-// Six kernels, each spread over the GPU by how many CTAs its sizes give:
+// Six kernels, or seven, each spread over the GPU by how many CTAs its sizes give:
 // adj_curv (warp per facet: scalars, areas, z, facet sums), adj_points (point
-// blocks x facet slices), adj_rows (CTA per relative lightcurve or block of
-// calibrated points: the slices' sums, model, residual, adjoint weights),
-// adj_facets (facet blocks x point blocks), adj_cols (blocks of facets: the
+// blocks x facet slices), adj_sums (CTA per block of points of one curve: the
+// slices' sums, model, columns of J; part of adj_rows where every curve is one
+// block), adj_rows (CTA per relative lightcurve or
+// block of calibrated points: residual, adjoint weights), adj_facets (facet blocks x point blocks), adj_cols (blocks of facets: the
 // F x C contraction), adj_out (CTA per free parameter).
 #include <cuda_runtime.h>
 #include <math.h>
@@ -284,18 +285,80 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
     for (int j = 0; j < kFixed + K; j++) W.pp[((size_t)j * W.nfs + blockIdx.y) * N + p] = acc[j];
 }
 
-// One item of the row list per CTA: a relative lightcurve, a block of
-// calibrated points, or (the last) the three convexity rows.  Per point the
-// slices' sums in slice order, then the model, the non-shape columns of J and
-// J v; per relative lightcurve ave = sum y and S = sum J v without v_1
-// (mrqcof.c:53-58, 92-104); per row the normalised model and J v, the residual,
-// u = W (y_obs - y') or W J' v, and the item's share of chi2; the adjoint
-// weights l.  (Five kernels before: 45 us of launches and of passes over the
-// rows at 20 000 points.)
+// A block of at most kAdjRowBlock points of one lightcurve, by kRowThreads
+// threads: the slices' sums in slice order, kRowThreads / kAdjRowBlock threads
+// per point, then a thread per point the model, the non-shape columns of J and
+// J v.
 template <int K>
+__device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W, const int4& item) {
+    __shared__ double sums[kFixed + K][kAdjRowBlock];
+    const int tid = threadIdx.x, N = P.n_points;
+    const double* x = W.misc;
+    const double cl = x[X_CL];
+    const int np = item.y - item.x, i0 = tid % kAdjRowBlock;
+    if (i0 < np)
+        for (int j = tid / kAdjRowBlock; j < kFixed + K; j += kRowThreads / kAdjRowBlock) {
+            const double* src = W.pp + (size_t)j * W.nfs * N + item.x + i0;
+            double v = 0;
+#pragma unroll 8
+            for (int k = 0; k < W.nfs; k++) v += src[(size_t)k * N];
+            sums[j][i0] = v;
+        }
+    __syncthreads();
+    if (tid >= np) return;
+    const int p = item.x + tid;
+    PointGeom G;
+    point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
+    double acc[kFixed + K];
+#pragma unroll
+    for (int j = 0; j < kFixed + K; j++) acc[j] = sums[j][tid];
+    const double br = acc[0], sc = G.scale, yy = br * sc;
+    double jn[9];
+    for (int k = 0; k < 3; k++) {
+        double v = 0;
+        for (int c = 0; c < 3; c++) v = fma(acc[3 + c], G.de[c][k], fma(acc[6 + c], G.de0[c][k], v));
+        jn[k] = sc * v;
+    }
+    jn[3] = br * G.dphp[0];
+    jn[4] = br * G.dphp[1];
+    jn[5] = br * G.dphp[2];
+    jn[6] = sc * acc[1] * cl;
+    jn[7] = sc * acc[2];
+    jn[8] = item.z ? 0.0 : yy;  // first shape coefficient
+    for (int j = 0; j < 9; j++) W.jns[(size_t)j * N + p] = jn[j];
+    W.y[p] = yy;
+    W.scale[p] = sc;
+#pragma unroll
+    for (int d = 0; d < K; d++) {
+        const double* v = W.dir + 9 * d;
+        double s = jn[8] * v[0];
+        for (int j = 0; j < 8; j++) s = fma(jn[j], v[1 + j], s);
+        W.jv[(size_t)d * N + p] = fma(sc, acc[kFixed + d], s);
+    }
+}
+
+// A block of points per CTA, where some relative lightcurve is longer than a
+// block: its own kernel, whose blocks spread over the GPU however long a
+// lightcurve is.  Inside adj_rows, a CTA per relative lightcurve, they took 3 us
+// each in turn: a gradient on one curve of 1000 / 5000 / 20 000 points and 800
+// facets 184 / 673 / 1313 us, 79 / 113 / 238 as a kernel of their own.  Where no
+// curve is longer, adj_rows forms the one block of its item itself and the
+// launch is saved: 60 calibrated points and 32 facets 58 against 62 us.
+template <int K>
+__global__ void __launch_bounds__(kRowThreads) adj_sums(const DevProblem* __restrict__ Pp, AdjWork W) {
+    block_sums<K>(*Pp, W, reinterpret_cast<const int4*>(Pp->ablocks)[blockIdx.x]);
+}
+
+// One item of the row list per CTA: a relative lightcurve, a block of
+// calibrated points, or (the last) the three convexity rows.  Per relative
+// lightcurve ave = sum y and S = sum J v without v_1 (mrqcof.c:53-58, 92-104);
+// per row the normalised model and J v, the residual, u = W (y_obs - y') or
+// W J' v, and the item's share of chi2; the adjoint weights l.  kOwnSums: the
+// item is one block, whose sums are formed here (see adj_sums).
+template <int K, bool kOwnSums>
 __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
-    __shared__ double red[32], sums[kFixed + K][kAdjRowBlock];
+    __shared__ double red[32];
     const int tid = threadIdx.x, N = P.n_points;
     const int4 item = reinterpret_cast<const int4*>(P.arows)[blockIdx.x];  // first row, last + 1, relative, points of the curve
     double* x = W.misc;
@@ -327,56 +390,20 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         if (tid == 0) W.x2part[blockIdx.x] = x2;
         return;
     }
+    if constexpr (kOwnSums) {
+        block_sums<K>(P, W, item);
+        __syncthreads();
+    }
     const bool rel = item.z != 0;
-    const double cl = x[X_CL];
     double sy = 0, sj[K];
 #pragma unroll
     for (int d = 0; d < K; d++) sj[d] = 0;
-    for (int p0 = item.x; p0 < item.y; p0 += kAdjRowBlock) {
-        // the slices' sums, in slice order, kRowThreads / kAdjRowBlock threads per point
-        const int np = min(kAdjRowBlock, item.y - p0), i0 = tid % kAdjRowBlock;
-        __syncthreads();
-        if (i0 < np)
-            for (int j = tid / kAdjRowBlock; j < kFixed + K; j += kRowThreads / kAdjRowBlock) {
-                const double* src = W.pp + (size_t)j * W.nfs * N + p0 + i0;
-                double v = 0;
-#pragma unroll 8
-                for (int k = 0; k < W.nfs; k++) v += src[(size_t)k * N];
-                sums[j][i0] = v;
-            }
-        __syncthreads();
-        if (tid >= np) continue;
-        const int p = p0 + tid;
-        PointGeom G;
-        point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
-        double acc[kFixed + K];
+    if (rel) {
+#pragma unroll 2
+        for (int p = item.x + tid; p < item.y; p += kRowThreads) {
+            sy += W.y[p];
 #pragma unroll
-        for (int j = 0; j < kFixed + K; j++) acc[j] = sums[j][tid];
-        const double br = acc[0], sc = G.scale, yy = br * sc;
-        double jn[9];
-        for (int k = 0; k < 3; k++) {
-            double v = 0;
-            for (int c = 0; c < 3; c++) v = fma(acc[3 + c], G.de[c][k], fma(acc[6 + c], G.de0[c][k], v));
-            jn[k] = sc * v;
-        }
-        jn[3] = br * G.dphp[0];
-        jn[4] = br * G.dphp[1];
-        jn[5] = br * G.dphp[2];
-        jn[6] = sc * acc[1] * cl;
-        jn[7] = sc * acc[2];
-        jn[8] = rel ? 0.0 : yy;  // first shape coefficient
-        for (int j = 0; j < 9; j++) W.jns[(size_t)j * N + p] = jn[j];
-        W.y[p] = yy;
-        W.scale[p] = sc;
-        sy += yy;
-#pragma unroll
-        for (int d = 0; d < K; d++) {
-            const double* v = W.dir + 9 * d;
-            double s = jn[8] * v[0];
-            for (int j = 0; j < 8; j++) s = fma(jn[j], v[1 + j], s);
-            s = fma(sc, acc[kFixed + d], s);
-            W.jv[(size_t)d * N + p] = s;
-            sj[d] += s;
+            for (int d = 0; d < K; d++) sj[d] += W.jv[(size_t)d * N + p];
         }
     }
     // coef of a row: L sigma / ave; rs is its sigma over the curve's first, one
@@ -582,7 +609,12 @@ cudaError_t launch(const DevProblem& P, const DevProblem* dP, double* work, cons
     W.mode = mode;
     adj_curv<K><<<W.ncurv, 32 * kCurvFacets, 0, s>>>(dP, W, args);
     adj_points<K><<<dim3(cdiv(P.n_points, kPtThreads), W.nfs), kPtThreads, 0, s>>>(dP, W);
-    adj_rows<K><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);
+    if (P.n_ablocks > 0) {
+        adj_sums<K><<<P.n_ablocks, kRowThreads, 0, s>>>(dP, W);
+        adj_rows<K, false><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);
+    } else {
+        adj_rows<K, true><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);
+    }
     adj_facets<K><<<dim3(cdiv(P.F, kFcThreads), W.npb), kFcThreads, 0, s>>>(dP, W);
     adj_cols<K><<<W.ncol, 128, 0, s>>>(dP, W);
     adj_out<K><<<dim3(P.mfit + 1, K), kOutThreads, 0, s>>>(dP, W, P.n_arows);

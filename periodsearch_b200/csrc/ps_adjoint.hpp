@@ -30,7 +30,7 @@ size_t adjoint_work_doubles(const DevProblem& P);
 constexpr int kAdjMiscChk = 33;
 constexpr int kAdjMiscSarea = 36;
 // Kernel launches of one launch_adjoint call.
-constexpr int kAdjointLaunches = 6;
+inline int adjoint_launches(const DevProblem& P) { return P.n_ablocks > 0 ? 7 : 6; }
 // chi2 into d_chi2; the result over the free parameters into d_out (mfit
 // values, kAdjDirs times mfit for kAdjUnits).
 cudaError_t launch_adjoint(const DevProblem& P, const DevProblem* dP, double* work, const AdjArgs& args, AdjMode mode,

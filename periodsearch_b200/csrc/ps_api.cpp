@@ -297,16 +297,20 @@ int upload_static(ps_ctx* c) {
         if (p.ia[i]) c->free_idx.push_back(i);
     std::vector<int> ints(lc);
     ints.insert(ints.end(), c->free_idx.begin(), c->free_idx.end());
-    // matrix-free form: antipodal facet pairs and the row items
+    // matrix-free form: antipodal facet pairs, the point blocks, the row items
     const size_t pair_at = ints.size();
     ints.insert(ints.end(), p.pairs->begin(), p.pairs->end());
     ints.resize((ints.size() + 3) & ~(size_t)3);  // items are read as int4
-    const size_t row_at = ints.size();
-    for (int i = 0; i < L; i++) {
-        const int block = p.lc_rel[i] ? p.lc_points[i] : psb::kAdjRowBlock;
+    auto cut = [&](int i, int block) {
         for (int r = lc_start[i]; r < lc_start[i + 1]; r += block)
             ints.insert(ints.end(), {r, std::min(r + block, lc_start[i + 1]), p.lc_rel[i], p.lc_points[i]});
-    }
+    };
+    const size_t block_at = ints.size();
+    bool longer = false;  // than a block: some relative lightcurve
+    for (int i = 0; i < L; i++) longer = longer || (p.lc_rel[i] && p.lc_points[i] > psb::kAdjRowBlock);
+    for (int i = 0; longer && i < L; i++) cut(i, psb::kAdjRowBlock);
+    const size_t row_at = ints.size();
+    for (int i = 0; i < L; i++) cut(i, p.lc_rel[i] ? p.lc_points[i] : psb::kAdjRowBlock);
     ints.insert(ints.end(), {N, N + 3, 0, 3});
     PSB_CUDA(c->d_lc.upload(ints, s));
     PSB_CUDA(c->d_queue.ensure(1));
@@ -338,6 +342,8 @@ int upload_static(ps_ctx* c) {
     d.lc_npts = c->d_lc.p + (L + 2) + (L + 1);
     d.free_idx = c->d_lc.p + lc.size();
     d.apair = p.pairs->empty() ? nullptr : c->d_lc.p + pair_at;
+    d.ablocks = c->d_lc.p + block_at;
+    d.n_ablocks = (int)((row_at - block_at) / 4);
     d.arows = c->d_lc.p + row_at;
     d.n_arows = (int)((ints.size() - row_at) / 4);
     d.fac = c->d_fac.p;
@@ -966,7 +972,7 @@ static int run_adjoint(ps_ctx* c, const double* a, const double* v, double* chi2
         for (int i = 0; i < d.mfit; i++) args.v[c->free_idx[i]] = v[i];
     PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, c->d_adj.p, args, v ? psb::kAdjProduct : psb::kAdjGradient, d_out,
                                  d_out + d.mfit, c->stream));
-    for (int k = 0; k < psb::kAdjointLaunches; k++) psb::count_launch();
+    for (int k = 0; k < psb::adjoint_launches(d); k++) psb::count_launch();
     double host[psb::kAdjMaxMa + 1];  // the result, then chi2
     PSB_CUDA(cudaMemcpyAsync(host, d_out, (d.mfit + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     PSB_CUDA(cudaStreamSynchronize(c->stream));
@@ -1065,7 +1071,7 @@ int jfree_eval(ps_ctx* c, const JfreeBufs& B, const double* a, bool full, std::v
     psb::AdjArgs args{};
     std::memcpy(args.a, a, d.ma * sizeof(double));
     PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, args, psb::kAdjGradient, B.beta, B.chi2, c->stream));
-    for (int k = 0; k < psb::kAdjointLaunches; k++) psb::count_launch();
+    for (int k = 0; k < psb::adjoint_launches(d); k++) psb::count_launch();
     // chck and the area sum depend on a only; the products write them again
     double host[4], x2 = 0;
     PSB_CUDA(cudaMemcpyAsync(host, B.work + psb::kAdjMiscChk, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1075,7 +1081,7 @@ int jfree_eval(ps_ctx* c, const JfreeBufs& B, const double* a, bool full, std::v
             for (int q = 0; q < psb::kAdjDirs; q++) args.unit[q] = k + q < mfit ? c->free_idx[k + q] : -1;
             PSB_CUDA(psb::launch_adjoint(d, c->d_dp.p, B.work, args, psb::kAdjUnits, B.alpha + (size_t)k * mfit,
                                          B.chi2 + 1, c->stream));
-            for (int q = 0; q < psb::kAdjointLaunches; q++) psb::count_launch();
+            for (int q = 0; q < psb::adjoint_launches(d); q++) psb::count_launch();
         }
         std::vector<double> cols((size_t)mfit * mfit);
         PSB_CUDA(cudaMemcpyAsync(cols.data(), B.alpha, cols.size() * sizeof(double), cudaMemcpyDeviceToHost,

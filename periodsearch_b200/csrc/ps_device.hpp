@@ -7,7 +7,7 @@
 
 namespace psb {
 
-constexpr int kAdjRowBlock = 64;  // rows of one item of the matrix-free row list
+constexpr int kAdjRowBlock = 64;  // points of one block of the matrix-free lists
 
 // Per-asteroid tables, all device pointers, 0-based.
 //  rows: n_points data rows (lightcurve order) followed by 3 convexity rows.
@@ -30,12 +30,14 @@ struct DevProblem {
     const int* free_idx; // [mfit] parameter index of each free parameter
     const double* cg_first;  // [C]
     const double* pole0;     // [10][2]: initial beta' and lambda [rad]
-    // matrix-free form: facets by antipodal pairs [F/2][2]; row items
-    // {first row, last + 1, relative, points of the lightcurve}: each relative
-    // lightcurve, blocks of the calibrated ones, the convexity rows
+    // matrix-free form: facets by antipodal pairs [F/2][2]; blocks of the points
+    // of each lightcurve {first, last + 1, relative, points of the lightcurve}, none
+    // if no relative lightcurve is longer than one; row items, likewise: each relative lightcurve, blocks of the calibrated
+    // ones, the convexity rows
     const int* apair;
+    const int* ablocks;
     const int* arows;
-    int n_arows;
+    int n_ablocks, n_arows;
     // tile shapes (ps_set_tiles / ps_autotune): the fast form's facets per
     // staged chunk and alpha rows per tile, and the points sorted together
     int fch, rt, sortseg;

@@ -2,6 +2,8 @@
 evaluation of the reference-order form (ps_mrqcof) on the same arrays: sigmas
 that differ within a curve, curves longer than the blocks the kernels take rows
 in.  Bars as for the other shapes: 1e-10 of what the sums add up from."""
+import time
+
 import numpy as np
 import pytest
 
@@ -59,3 +61,29 @@ def _check(native, desc, seed):
                                                ([(0, 30), (1, 1), (1, 300)], 4, 5)])
 def test_sigma_varying_within_a_curve(native, curves, lmax, nrows):
     _check(native, _desc(3, curves, lmax, nrows, True), 4)
+
+
+@pytest.mark.parametrize("curves,lmax,nrows", [([(1, 64)], 2, 3), ([(0, 64), (1, 129)], 3, 4),
+                                               ([(1, 255), (1, 256), (0, 257), (1, 700)], 4, 5), ([(1, 5000)], 6, 10)])
+def test_curves_longer_than_a_block(native, curves, lmax, nrows):
+    _check(native, _desc(5, curves, lmax, nrows, False), 6)
+
+
+def test_time_of_a_long_relative_curve(native):
+    """The rows of one long relative lightcurve spread over the GPU like those of
+    calibrated points: a gradient costs less than twice as much on it."""
+    us = {}
+    for rel in (0, 1):
+        g = native.PeriodSearch(desc=_desc(7, [(rel, 20000)], 6, 10, False), form=native.PS_FORM_FAST)
+        g.set_conw_r(0.4)
+        a = np.concatenate([g.array("cg_first"), [0.4, 1.0, 24 * 2 * np.pi * g.freq_start, 0.5, 0.1, -0.5, np.log(0.1), 1.0]])
+        g.chi2_grad(a)
+        t = []
+        for _ in range(9):
+            t0 = time.perf_counter()
+            g.chi2_grad(a)
+            t.append(time.perf_counter() - t0)
+        us[rel] = 1e6 * sorted(t)[2]
+        g.close()
+    print(f"gradient, 20 000 points, 800 facets: {us[0]:.0f} us calibrated, {us[1]:.0f} us on one relative curve")
+    assert us[1] < 2 * us[0]
