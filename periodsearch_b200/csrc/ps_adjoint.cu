@@ -59,7 +59,7 @@ enum { X_B = 0, X_D = 9, X_CL = 27, X_CLS = 28, X_OMG = 29, X_P1 = 30, X_P2 = 31
        X_SAREA = kAdjMiscSarea, X_UC = 40, X_N = X_UC + 3 * kAdjDirs };
 
 // Device work arrays of one evaluation, carved from one buffer of
-// adjoint_work_doubles(P) doubles; K directions.
+// adjoint_work_doubles doubles; K directions.
 struct AdjWork {
     double* misc;    // scalars, then u of the convexity rows [K][3]
     double* dir;     // [K][9]: v of the first shape coefficient, then of the non-shape parameters
@@ -623,9 +623,11 @@ cudaError_t launch(const DevProblem& P, const DevProblem* dP, double* work, cons
 
 }  // namespace
 
-size_t adjoint_work_doubles(const DevProblem& P) {
+size_t adjoint_work_doubles(const DevProblem& P, bool batched) {
     AdjWork W{};
-    const size_t one = carve<1>(P, nullptr, W), all = carve<kAdjDirs>(P, nullptr, W);
+    const size_t one = carve<1>(P, nullptr, W);
+    if (!batched) return one;
+    const size_t all = carve<kAdjDirs>(P, nullptr, W);
     return one > all ? one : all;
 }
 

@@ -24,7 +24,9 @@ enum AdjMode {
     kAdjUnits      // J^T W (J e) for kAdjDirs unit vectors e
 };
 
-size_t adjoint_work_doubles(const DevProblem& P);
+// Doubles of work memory of a gradient or product; batched: of those and a batch
+// of kAdjDirs products, about twice as many.
+size_t adjoint_work_doubles(const DevProblem& P, bool batched);
 // Scalars of the last evaluation at work: the convexity residuals chck (3) at
 // kAdjMiscChk, the facet-area sum after them.
 constexpr int kAdjMiscChk = 33;

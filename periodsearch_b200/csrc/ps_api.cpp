@@ -963,7 +963,7 @@ static int run_adjoint(ps_ctx* c, const double* a, const double* v, double* chi2
     if (!a) return fail(PS_ERR_ARG, "null parameter vector");
     PSB_CUDA(cudaSetDevice(c->device));
     const psb::DevProblem& d = c->dp;
-    const size_t work = psb::adjoint_work_doubles(d);
+    const size_t work = psb::adjoint_work_doubles(d, false);
     PSB_CUDA(c->d_adj.ensure(work + d.mfit + 1));
     double* d_out = c->d_adj.p + work;
     psb::AdjArgs args{};
@@ -1053,7 +1053,7 @@ JfreeBufs jfree_bufs(ps_ctx* c) {
     const psb::DevProblem& d = c->dp;
     JfreeBufs B;
     B.work = c->d_adj.p;
-    B.alpha = B.work + psb::adjoint_work_doubles(d);
+    B.alpha = B.work + psb::adjoint_work_doubles(d, true);
     B.beta = B.alpha + jfree_columns(d.mfit) * d.mfit;
     B.chi2 = B.beta + d.mfit;
     return B;
@@ -1116,7 +1116,7 @@ int ps_fit_jfree(ps_ctx* c, double freq, int pole, ps_fit_result* out, double* c
     PSB_CUDA(cudaSetDevice(c->device));
     const psb::DevProblem& d = c->dp;
     const int ma = d.ma, mfit = d.mfit, C = d.C;
-    PSB_CUDA(c->d_adj.ensure(psb::adjoint_work_doubles(d) + jfree_columns(mfit) * mfit + mfit + 2));
+    PSB_CUDA(c->d_adj.ensure(psb::adjoint_work_doubles(d, true) + jfree_columns(mfit) * mfit + mfit + 2));
     const JfreeBufs B = jfree_bufs(c);
     std::vector<double> cg(ma), atry(ma), alpha, beta, covar, da;
     psb::initial_parameters(c->prob, freq, pole, cg.data());

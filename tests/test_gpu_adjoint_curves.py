@@ -87,3 +87,20 @@ def test_time_of_a_long_relative_curve(native):
         g.close()
     print(f"gradient, 20 000 points, 800 facets: {us[0]:.0f} us calibrated, {us[1]:.0f} us on one relative curve")
     assert us[1] < 2 * us[0]
+
+
+def test_work_memory_of_a_gradient(native):
+    """A gradient takes work memory for one direction (16.5 MB at 20 000 points
+    and 2048 facets), not for the batch of eight of a Jacobian-free fit (38 MB)."""
+    torch = pytest.importorskip("torch")
+    taken = []
+    for points, nrows in ((60, 3), (20000, 16)):  # the first loads the kernels
+        g = native.PeriodSearch(desc=_desc(8, [(0, points)], 3, nrows, False), form=native.PS_FORM_FAST)
+        g.set_conw_r(0.4)
+        a = np.concatenate([g.array("cg_first"), [0.4, 1.0, 24 * 2 * np.pi * g.freq_start, 0.5, 0.1, -0.5, np.log(0.1), 1.0]])
+        native.load_library().ps_release_cached_memory()
+        free = torch.cuda.mem_get_info()[0]
+        g.chi2_grad(a)
+        taken.append(free - torch.cuda.mem_get_info()[0])
+        g.close()
+    assert taken[1] < 24 << 20, taken
