@@ -52,9 +52,9 @@ __device__ __forceinline__ double rcp_nearest(double x) {
 // q + y (a - d q), which rounds correctly: it is off by less than
 // 2^-53 |a / d - q| before its rounding, and where a / d lies so close to a middle
 // that this could matter, q is one of its two neighbours.  a and d of ordinary
-// size (no overflow, underflow or special value anywhere on the way; a may be
-// zero).  No branch and no call, unlike the division, so several run side by
-// side.
+// size (plain_numerator: no overflow, underflow or special value anywhere on the
+// way; zero is fine).  No branch and no call, unlike the division, so several run
+// side by side.
 struct QuotientsBy {
     double d, y;
     __device__ __forceinline__ explicit QuotientsBy(double divisor) : d(divisor), y(rcp_nearest(divisor)) {}
@@ -62,7 +62,17 @@ struct QuotientsBy {
         const double q = a * y;
         return fma(fma(-d, q, a), y, q);
     }
+    // any a: scaled by a power of two where it is out of the ordinary (a
+    // subnormal quotient is within its spacing of the division's)
+    __device__ __forceinline__ double of_any(double a) const {
+        if (!isfinite(a)) return a * y;
+        const double s = fabs(a) > 1.0 ? 0x1p-600 : 0x1p600;
+        return of(a * s) * (1.0 / s);
+    }
 };
+
+// Whether QuotientsBy::of takes a over divisors in (2e-8, 4].
+__device__ __forceinline__ bool plain_numerator(double a) { return a == 0.0 || (fabs(a) > 1e-200 && fabs(a) < 1e200); }
 
 // blmatrix.c:9-46.  B[i*3+j] = Blmat[i+1][j+1]; D[(d*3+i)*3+j] = Dblm[d+1][i+1][j+1].
 __device__ void blmatrix(double bet, double lam, double* B, double* D) {

@@ -805,8 +805,7 @@ __device__ void model_pass(const DevProblem& P, const double* a, double* g, doub
     eval_scalars(a, P.C, B, D, misc);
     curv_phase(P, a, g, area, false);
     __syncthreads();
-    const double cls = misc[M_CLS];
-    if (kFast || (fabs(cls) > 1e-200 && fabs(cls) < 1e200))
+    if (kFast || plain_numerator(misc[M_CLS]))
         model_points<kFast, true>(P, area, misc, B, work, perm, sorted, yt);
     else
         model_points<kFast, false>(P, area, misc, B, work, perm, sorted, yt);
@@ -874,11 +873,13 @@ __device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, i
 // 6.3 -> 5.8 ms, the pre-pass and 400 fits of 500 points 104 -> 97 ms; 290 fits
 // of 500 points and 25 coefficients 34.3 -> 32.3, of 700 and 36 60 -> 58; at 49
 // coefficients 249 -> 256.
-// `p`: the thread's point, -1 for none.  first: also the facet sums.  want_cl, all: also the columns of the
-// Lambert coefficient, of the (never fitted) Lommel-Seeliger one.
-template <int NCB, int H, int kFirst, int kCount>
+// `p`: the thread's point, -1 for none.  first: also the facet sums.  want_cl:
+// also the column of the Lambert coefficient.  kAll: also that of the
+// Lommel-Seeliger coefficient, which no fit varies, and any value of it (fits
+// hold it at 1, and the test of its size costs them 1.5 %).
+template <int NCB, int H, int kFirst, int kCount, bool kAll>
 __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, bool first, bool ordinary,
-                                      bool want_cl, bool all, double* Jt, double* yt) {
+                                      bool want_cl, double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const DevProblem& P = *Pp;
     const Layout L = make_layout(P);
@@ -898,7 +899,7 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
     const int tid = threadIdx.x;
     const int F = P.F, C = P.C, npad = P.npad;
     const double cl = misc[M_CL], cls = misc[M_CLS];
-    const bool finite = isfinite(cls);  // cls / d is cls where it is not
+    const bool plain = !kAll || plain_numerator(cls);
     constexpr int c0 = H == 0 ? 0 : 2;  // the rotation derivative both halves keep
     // this point's derivative vectors in shared memory ([vector][slot]: the
     // loads of a warp are consecutive): H = 0 columns 0 and 1 of de, de0
@@ -987,7 +988,7 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
                 const double dnom = vis[u] ? mu + mu0 : 1.0;
                 const QuotientsBy by(dnom);
                 const double q0 = by.of(mu0), q1 = by.of(mu);
-                sv[u] = mu * mu0 * (cl + (finite ? by.of(cls) : cls * by.y));
+                sv[u] = mu * mu0 * (cl + (plain ? by.of(cls) : by.of_any(cls)));
                 dsmu[u] = cls * (q0 * q0) + cl * mu0;
                 dsmu0[u] = cls * (q1 * q1) + cl * mu;
                 cmu[u] = mu;
@@ -1024,7 +1025,7 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
                     } else if (want_cl && vis[u]) {
                         const double ar = fq[5 * u + 3];
                         a0 = a0 + cmu[u] * cmu0[u] * ar;
-                        if (all) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
+                        if (kAll) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
                     }
                 }
                 continue;
@@ -1050,7 +1051,7 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
                     a2 = a2 + ar * (dsmu[u] * sum + dsmu0[u] * sum0);
                 } else {
                     if (want_cl) a0 = a0 + cmu[u] * cmu0[u] * ar;
-                    if (all) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
+                    if (kAll) a2 = a2 + ar * cmu[u] * cmu0[u] / (cmu[u] + cmu0[u]);
                 }
             }
         }
@@ -1091,20 +1092,20 @@ __device__ __noinline__ void ref_pass(const DevProblem* __restrict__ Pp, int p, 
 // Both halves of a pass over kTotal coefficients.  Half 0's extra rotation
 // derivative and brightness sum are 17 operations per pair, the shape sums 2
 // each, so half 1 takes eight more of them.
-template <int NCB, int kTotal>
+template <int NCB, int kTotal, bool kAll>
 __device__ __forceinline__ void ref_halves(const DevProblem* __restrict__ Pp, int h, int p, bool first, bool ordinary,
-                                           bool want_cl, bool all, double* Jt, double* yt) {
+                                           bool want_cl, double* Jt, double* yt) {
     constexpr int k0 = kTotal > 9 ? (kTotal - 8) / 2 & ~1 : 0;  // even: dg is read in pairs
     if (h == 0)
-        ref_pass<NCB, 0, 0, k0>(Pp, p, first, ordinary, want_cl, all, Jt, yt);
+        ref_pass<NCB, 0, 0, k0, kAll>(Pp, p, first, ordinary, want_cl, Jt, yt);
     else
-        ref_pass<NCB, 1, k0, kTotal - k0>(Pp, p, first, ordinary, want_cl, all, Jt, yt);
+        ref_pass<NCB, 1, k0, kTotal - k0, kAll>(Pp, p, first, ordinary, want_cl, Jt, yt);
 }
 
 // ref_pass over every data point, in segments sorted by viewing direction.
-template <int NCB>
+template <int NCB, bool kAll>
 __device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp, double* sm, const Layout& L,
-                                               bool ordinary, bool all, double* Jt, double* yt) {
+                                               bool ordinary, double* Jt, double* yt) {
     constexpr int kPts = kThreads / 2;
     const DevProblem& P = *Pp;
     const int tid = threadIdx.x, h = tid / kPts, pl = tid - h * kPts;
@@ -1112,7 +1113,7 @@ __device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp
     const double* misc = sm + L.misc;
     double* work = sm + L.work;
     int* perm = (int*)(sm + L.perm);
-    const bool want_cl = all || P.free_idx[P.mfit - 1] >= P.C + 6;
+    const bool want_cl = kAll || P.free_idx[P.mfit - 1] >= P.C + 6;
     for (int s0 = 0; s0 < P.n_points; s0 += P.sortseg) {
         const int seg = min(P.sortseg, P.n_points - s0);
         __syncthreads();
@@ -1122,9 +1123,9 @@ __device__ __forceinline__ void point_loop_ref(const DevProblem* __restrict__ Pp
             const bool first = s0 == 0 && base == 0;
             // C = 1 mod 8 for every even lmax = mmax: no sums for the padding
             if (P.C > NCB - 7)
-                ref_halves<NCB, NCB>(Pp, h, p, first, ordinary, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB, kAll>(Pp, h, p, first, ordinary, want_cl, Jt, yt);
             else
-                ref_halves<NCB, NCB - 7>(Pp, h, p, first, ordinary, want_cl, all, Jt, yt);
+                ref_halves<NCB, NCB - 7, kAll>(Pp, h, p, first, ordinary, want_cl, Jt, yt);
         }
     }
 }
@@ -1225,9 +1226,11 @@ __device__ __noinline__ void ref_alpha(const DevProblem* __restrict__ Pp, int al
     }
 }
 
-template <int NCB, bool kFast>
+// kAll: every column of J, at any scattering coefficients (the reference-order
+// form; the fast form always).
+template <int NCB, bool kFast, bool kAll>
 __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_off, int alpha_off, int beta_off,
-                                      bool all, double* Jt, double* yt) {
+                                      double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const double* a = sm + a_off;
     double* alpha_out = sm + alpha_off;
@@ -1256,7 +1259,7 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
             point_loop_fast<NCB, false>(Pp, Jt, yt);
         }
     } else {
-        point_loop_ref<NCB>(Pp, sm, L, ordinary, all, Jt, yt);
+        point_loop_ref<NCB, kAll>(Pp, sm, L, ordinary, Jt, yt);
     }
     __syncthreads();
     // convexity rows (conv.c:12-29): y = residual, J = dres for the shape
@@ -1425,7 +1428,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
         while (((niter < P.n_iter_max) && (iter_diff > P.iter_diff_max)) || (niter < P.n_iter_min)) {
             if (alamda < 0) {
                 alamda = P.alamda_start;
-                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), false, Jt, yt);
+                evaluate<NCB, kFast, false>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), Jt, yt);
                 ochisq = misc[M_CHISQ];
                 cur0 = misc[M_CHK0];
                 cur1 = misc[M_CHK0 + 1];
@@ -1435,7 +1438,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
             } else if (j_stale) {
                 // alpha and beta at the point accepted last (its chi2, chck and
                 // area sum came from the model-only evaluation and are kept)
-                evaluate<NCB, kFast>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), false, Jt, yt);
+                evaluate<NCB, kFast, false>(Pp, (int)(cg - sm), (int)(alpha - sm), (int)(beta - sm), Jt, yt);
                 j_stale = false;
             }
             for (int idx = tid; idx < mfit * mfit; idx += kThreads) {
@@ -1531,7 +1534,7 @@ __global__ void __launch_bounds__(kThreads, 1) eval_kernel(const DevProblem* __r
     alpha_jobs(P.mfit, (int*)(sm + L.ent));
     for (int i = tid; i < P.ma; i += kThreads) cg[i] = E.a[i];
     __syncthreads();
-    evaluate<NCB, kFast>(Pp, L.cg, L.alpha, L.beta, true, Jt, yt);
+    evaluate<NCB, kFast, !kFast>(Pp, L.cg, L.alpha, L.beta, Jt, yt);
     for (int i = tid; i < P.mfit * P.mfit; i += kThreads) E.alpha[i] = sm[L.alpha + i];
     for (int i = tid; i < P.mfit; i += kThreads) E.beta[i] = sm[L.beta + i];
     if (tid == 0) E.chisq[0] = sm[L.misc + M_CHISQ];

@@ -8,7 +8,7 @@ __global__ void quotients(const double* a, const double* d, int n, double* out) 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const psb::fitcommon::QuotientsBy by(d[i]);
-    out[i] = by.of(a[i]);
+    out[i] = psb::fitcommon::plain_numerator(a[i]) ? by.of(a[i]) : by.of_any(a[i]);
     out[n + i] = a[i] / d[i];
     out[2 * n + i] = by.y;
     out[3 * n + i] = 1.0 / d[i];

@@ -76,6 +76,22 @@ def test_random_operands():
         assert np.max(np.abs(y_newton - y_ref) / np.spacing(y_ref)) <= 1
 
 
+def test_numerators_out_of_the_ordinary():
+    """Beyond 1e200 in size or below 1e-200, infinite, not a number: the division's
+    quotient, a subnormal one to its spacing."""
+    rng = np.random.default_rng(3)
+    d = _divisors(rng, 1 << 16)
+    tiny, huge = 10.0 ** rng.uniform(-323, -200, d.size), 10.0 ** rng.uniform(200, 308, d.size)
+    for a in (tiny, -tiny, huge, -huge):
+        q, q_ref, *_ = _quotients(a, d)
+        sub = np.abs(q_ref) < 2.3e-308
+        assert np.array_equal(q[~sub], q_ref[~sub])
+        assert np.abs(q[sub] - q_ref[sub]).max(initial=0.0) <= 5e-324
+    for a in (np.inf, -np.inf, np.nan):
+        q, q_ref, *_ = _quotients(np.full(d.size, a), d)
+        assert np.array_equal(q, q_ref, equal_nan=True)
+
+
 def test_quotients_near_a_middle():
     rng = np.random.default_rng(2)
     a, d = _middles(rng, 200_000)
