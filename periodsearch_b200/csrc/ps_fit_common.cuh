@@ -106,6 +106,18 @@ __device__ void blmatrix(double bet, double lam, double* B, double* D) {
     D[17] = 0;
 }
 
+// Loops over pairs without a branch give a facet that is not seen area 0 times
+// its terms.  Those are finite at these scattering coefficients ...
+__host__ __device__ __forceinline__ bool ordinary_scattering(double cl, double cls) {
+    return fabs(cl) < 1e200 && fabs(cls) < 1e200;
+}
+
+// ... and for directions that are numbers; a point with others sees no facet, as
+// none of its comparisons holds.
+__device__ __forceinline__ bool visible_geometry(const double* e, const double* e0) {
+    return fabs(e[0]) + fabs(e[1]) + fabs(e[2]) + fabs(e0[0]) + fabs(e0[1]) + fabs(e0[2]) < 1e200;
+}
+
 struct PointGeom {
     double e[3], e0[3];
     double de[3][3], de0[3][3];  // [component][derivative], bright.c:41-53

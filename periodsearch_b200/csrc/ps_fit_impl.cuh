@@ -264,7 +264,8 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // 8-column tile would carry a single coefficient, so coefficient C - 1 is
 // summed per lane on the FP64 pipe (one FMA per visible pair) and the MMA
 // sequence covers the first NCB - 8 columns.
-template <int NCB, bool kX1>
+// kMasked: at scattering coefficients that are not ordinary_scattering.
+template <int NCB, bool kX1, bool kMasked>
 __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, double* Jt, double* yt) {
     extern __shared__ __align__(16) double sm[];
     const DevProblem& P = *Pp;
@@ -313,6 +314,8 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
                     e[c] = G.e[c];
                     e0[c] = G.e0[c];
                 }
+                if (!visible_geometry(e, e0))
+                    e[0] = e[1] = e[2] = e0[0] = e0[1] = e0[2] = 0;
             }
             double acc[NT][2];
             double br = 0, T[3] = {0, 0, 0}, S[3] = {0, 0, 0}, s_cl = 0, s_cls = 0, x1 = 0;
@@ -353,7 +356,8 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
                 // Facets past F (zero rows in the staged chunk, zero area) and
                 // inactive lanes (e = e0 = 0) have mu = mu0 = 0: not visible.
                 // A step whose pairs some lane sees runs without a branch: a facet the
-                // lane does not see counts with area 0, which leaves every sum as it is.
+                // lane does not see counts with area 0, which leaves every sum as it is
+                // while its terms are finite (kMasked: zeros in their place).
                 for (int j = 0; j < nf; j += 4) {
                     const int ff = j + q;
                     const double2 nxy = *reinterpret_cast<const double2*>(fb + ff * 4);
@@ -364,11 +368,13 @@ __device__ __noinline__ void point_loop_fast(const DevProblem* __restrict__ Pp, 
                     if (!__any_sync(full, vis)) continue;
                     const double ar = vis ? area[f0 + ff] : 0.0;
                     const double r = rcp_nearest(vis ? mu + mu0 : 1.0);
-                    const double av = ar * (mu * mu0 * fma(cls, r, cl));
+                    double av = ar * (mu * mu0 * fma(cls, r, cl));
+                    if (kMasked && !vis) av = 0;
                     br = __dadd_rn(br, av);
                     const double q0 = mu0 * r, q1 = mu * r;
-                    const double w = ar * fma(cls * q0, q0, cl * mu0);
-                    const double w0 = ar * fma(cls * q1, q1, cl * mu);
+                    double w = ar * fma(cls * q0, q0, cl * mu0);
+                    double w0 = ar * fma(cls * q1, q1, cl * mu);
+                    if (kMasked && !vis) w = w0 = 0;
                     T[0] = fma(w, nxy.x, T[0]);
                     T[1] = fma(w, nxy.y, T[1]);
                     T[2] = fma(w, nz, T[2]);
@@ -1226,8 +1232,8 @@ __device__ __noinline__ void ref_alpha(const DevProblem* __restrict__ Pp, int al
     }
 }
 
-// kAll: every column of J, at any scattering coefficients (the reference-order
-// form; the fast form always).
+// kAll: every column of J, at any scattering coefficients; fits accept a step
+// only to finite ones.
 template <int NCB, bool kFast, bool kAll>
 __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_off, int alpha_off, int beta_off,
                                       double* Jt, double* yt) {
@@ -1250,13 +1256,17 @@ __device__ __noinline__ void evaluate(const DevProblem* __restrict__ Pp, int a_o
     eval_scalars(a, C, B, D, misc);
     const bool ordinary = __syncthreads_and(curv_phase(P, a, g, area));
     if constexpr (kFast) {
-        if constexpr (NCB >= 16) {
-            if (C == NCB - 7)
-                point_loop_fast<NCB, true>(Pp, Jt, yt);
+        constexpr bool kCanX1 = NCB >= 16;
+        const bool x1 = kCanX1 && C == NCB - 7;
+        if (kAll && !ordinary_scattering(misc[M_CL], misc[M_CLS])) {
+            if (x1)
+                point_loop_fast<NCB, kCanX1, kAll>(Pp, Jt, yt);
             else
-                point_loop_fast<NCB, false>(Pp, Jt, yt);
+                point_loop_fast<NCB, false, kAll>(Pp, Jt, yt);
+        } else if (x1) {
+            point_loop_fast<NCB, kCanX1, false>(Pp, Jt, yt);
         } else {
-            point_loop_fast<NCB, false>(Pp, Jt, yt);
+            point_loop_fast<NCB, false, false>(Pp, Jt, yt);
         }
     } else {
         point_loop_ref<NCB, kAll>(Pp, sm, L, ordinary, Jt, yt);
@@ -1534,7 +1544,7 @@ __global__ void __launch_bounds__(kThreads, 1) eval_kernel(const DevProblem* __r
     alpha_jobs(P.mfit, (int*)(sm + L.ent));
     for (int i = tid; i < P.ma; i += kThreads) cg[i] = E.a[i];
     __syncthreads();
-    evaluate<NCB, kFast, !kFast>(Pp, L.cg, L.alpha, L.beta, Jt, yt);
+    evaluate<NCB, kFast, true>(Pp, L.cg, L.alpha, L.beta, Jt, yt);
     for (int i = tid; i < P.mfit * P.mfit; i += kThreads) E.alpha[i] = sm[L.alpha + i];
     for (int i = tid; i < P.mfit; i += kThreads) E.beta[i] = sm[L.beta + i];
     if (tid == 0) E.chisq[0] = sm[L.misc + M_CHISQ];

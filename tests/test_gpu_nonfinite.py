@@ -1,0 +1,47 @@
+"""Infinite and undefined values: what they touched before the loops over pairs
+lost their branches, and nothing else.  A Lambert coefficient exp(a) that
+overflows makes a point's brightness infinite if it sees a facet and leaves it
+zero if it sees none (opposite Sun and Earth); a point whose time is not a number
+sees none."""
+import numpy as np
+import pytest
+
+from test_gpu_adjoint_curves import _desc
+
+pytestmark = pytest.mark.gpu
+
+DARK, LOST = 7, 40  # a point opposite the Sun; one without a time
+N = 150
+
+
+def _problem(lmax, nrows, lost, **more):
+    d = _desc(11, [(0, N)], lmax, nrows, False)
+    d["ee0"][DARK] = -d["ee"][DARK]
+    if lost:
+        d["tim"][LOST] = np.nan
+    return dict(d, **more)
+
+
+def _open(native, form, desc):
+    g = native.PeriodSearch(desc=desc, form={"fp64": native.PS_FORM_FP64, "fast": native.PS_FORM_FAST}[form])
+    g.set_conw_r(0.4)
+    return g, np.concatenate([g.array("cg_first"), [0.4, 1.0, 24 * 2 * np.pi * g.freq_start, 0.5, 0.1, -0.5, np.log(0.1), 1.0]])
+
+
+# coefficient counts with and without the column on the FP64 pipe
+@pytest.mark.parametrize("form", ["fp64", "fast"])
+@pytest.mark.parametrize("lmax,nrows", [(1, 3), (2, 4), (4, 5), (8, 9)])
+def test_rows(native, form, lmax, nrows):
+    g, a = _open(native, form, _problem(lmax, nrows, True))
+    C = g.ncoef
+    seen = np.ones(N, bool)
+    seen[[DARK, LOST]] = False
+    y, J = g.model(a)
+    assert np.all(np.isfinite(y)) and np.all(y[:N][seen] > 0) and np.all(y[:N][~seen] == 0)
+    assert np.all(np.isfinite(J[:N][seen])) and np.all(np.isfinite(J[DARK]))
+    for log_cl, cls in ((800.0, 1.0), (-2.0, np.inf), (705.0, 1e308)):
+        a[C + 6], a[C + 7] = log_cl, cls
+        y, J = g.model(a)
+        assert np.all(np.isposinf(y[:N][seen])) and np.all(y[:N][~seen] == 0), (log_cl, cls)
+        assert np.all(np.isposinf(J[:N][seen, 0])) and np.all(J[:N][~seen, :C] == 0), (log_cl, cls)
+    g.close()
