@@ -661,33 +661,17 @@ __device__ __forceinline__ void chi2_rows(const DevProblem& P, const double* yt,
     }
 }
 
-// The model alone at parameters a: what the LM step's accept/reject test and
-// the stop rule read from mrqcof at a trial point -- chi2, the convexity
-// residuals chck (conv.c:22-27) and the facet-area sum -- without the
-// Jacobian or alpha/beta.  curv, the brightness of every point
-// (bright.c:54-76, 106-125 without the derivative terms), the convexity
-// rows, the relative-lightcurve normalisation of the model (mrqcof.c:53-58,
-// 92-104) and chi2, with the operations and sum orders of evaluate(), so
-// that in the reference-order form every value is bit-identical to the one
-// evaluate() gives at the same point.  The model goes to yt; Jt is not
-// touched.  Thread per data point, facet normals staged in chunks of kMf, four
-// facets at a time (model_facets).
-// Buffers (shared memory): g, area [F] (area is not padded past F here);
-// misc and B/D (blmatrix) as in evaluate(); work >= max(sortseg, 4 kMf,
-// kThreads) doubles, 16-byte aligned; perm sortseg ints.  sorted: perm still
-// holds the points in the order of a nearby viewing geometry (any order gives
-// the same sums).  Used by the FP64 fit kernels (evaluate_model) and the
-// mixed-precision one.
 // Facets [0, kU) of `nrm` ({nx, ny, nz, Area}, zeros where there is no facet)
 // for one point per lane: the terms of all kU without a branch, so that their
 // chains run side by side, then the sum in facet order.  A facet that the lane
-// does not see adds Area 0 times a finite value, which leaves the sum as it is.
-// kPlain: see QuotientsBy.  Bound by the latency of one pair's chain: a warp that
+// does not see adds Area 0 times its term, which leaves the sum as it is: a fit's
+// Lommel-Seeliger coefficient is 1, and where its Lambert coefficient overflows
+// the trial's chi2 is infinite or no number and rejected either way.  Bound by the latency of one pair's chain: a warp that
 // took the facets one by one, with the IEEE division's branch, spent 470 cycles
 // on each at 118 points (one warp per scheduler), 135 000 of a step's 430 000.
 // Four at a time: one fit of 118 points and 288 facets 9.7 -> 7.6 ms, 600 fits
 // of 760 points and 800 facets 339 -> 314 ms.
-template <bool kFast, bool kPlain, int kU>
+template <bool kFast, int kU>
 __device__ __forceinline__ void model_facets(const double4* nrm, const double* e, const double* e0, double cl, double cls,
                                              double& br) {
     double mu[kU], mu0[kU], w[kU];
@@ -709,7 +693,7 @@ __device__ __forceinline__ void model_facets(const double4* nrm, const double* e
             const double r = rcp_newton(dnom);
             mu[u] = mu[u] * mu0[u] * fma(cls, r, cl);
         } else {
-            const double s = mu[u] * mu0[u] * (cl + (kPlain ? QuotientsBy(dnom).of(cls) : cls / dnom));
+            const double s = mu[u] * mu0[u] * (cl + QuotientsBy(dnom).of(cls));
             mu[u] = w[u] * s;
         }
     }
@@ -724,7 +708,7 @@ __device__ __forceinline__ void model_facets(const double4* nrm, const double* e
 
 // The brightness of every data point to yt, with chck and the facet-area sum
 // on the way (four lanes of the last warp, facets in order).
-template <bool kFast, bool kPlain>
+template <bool kFast>
 __device__ __forceinline__ void model_points(const DevProblem& P, const double* area, double* misc, const double* B,
                                              double* work, int* perm, bool sorted, double* yt) {
     constexpr int kU = 4;  // facets at a time
@@ -756,6 +740,7 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
                         ej[j][c] = G.e[c];
                         fj[j][c] = G.e0[c];
                     }
+                    if (!visible_geometry(ej[j], fj[j])) ej[j][0] = ej[j][1] = ej[j][2] = fj[j][0] = fj[j][1] = fj[j][2] = 0;
                     sc[j] = G.scale;
                 }
             }
@@ -786,7 +771,7 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
                     // a warp without points in this slot has nothing to do
                     if (j >= k || base + j * kThreads + (tid & ~31) >= seg) continue;
                     for (int ff = 0; ff < nf; ff += kU)
-                        model_facets<kFast, kPlain, kU>(nrm + ff, ej[j], fj[j], cl, cls, br[j]);
+                        model_facets<kFast, kU>(nrm + ff, ej[j], fj[j], cl, cls, br[j]);
                 }
             }
 #pragma unroll
@@ -799,6 +784,23 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
     if (job >= 0 && job < 4) misc[job < 3 ? M_CHK0 + job : M_SAREA] = sum;
 }
 
+// The model alone at parameters a: what the LM step's accept/reject test and
+// the stop rule read from mrqcof at a trial point -- chi2, the convexity
+// residuals chck (conv.c:22-27) and the facet-area sum -- without the
+// Jacobian or alpha/beta.  curv, the brightness of every point
+// (bright.c:54-76, 106-125 without the derivative terms), the convexity
+// rows, the relative-lightcurve normalisation of the model (mrqcof.c:53-58,
+// 92-104) and chi2, with the operations and sum orders of evaluate(), so
+// that in the reference-order form every value is bit-identical to the one
+// evaluate() gives at the same point.  The model goes to yt; Jt is not
+// touched.  Thread per data point, facet normals staged in chunks of kMf, four
+// facets at a time (model_facets).
+// Buffers (shared memory): g, area [F] (area is not padded past F here);
+// misc and B/D (blmatrix) as in evaluate(); work >= max(sortseg, 4 kMf,
+// kThreads) doubles, 16-byte aligned; perm sortseg ints.  sorted: perm still
+// holds the points in the order of a nearby viewing geometry (any order gives
+// the same sums).  Used by the FP64 fit kernels (evaluate_model) and the
+// mixed-precision one.
 template <bool kFast>
 __device__ void model_pass(const DevProblem& P, const double* a, double* g, double* area, double* misc, double* B,
                            double* D, double* work, int* perm, bool sorted, double* yt) {
@@ -811,10 +813,7 @@ __device__ void model_pass(const DevProblem& P, const double* a, double* g, doub
     eval_scalars(a, P.C, B, D, misc);
     curv_phase(P, a, g, area, false);
     __syncthreads();
-    if (kFast || plain_numerator(misc[M_CLS]))
-        model_points<kFast, true>(P, area, misc, B, work, perm, sorted, yt);
-    else
-        model_points<kFast, false>(P, area, misc, B, work, perm, sorted, yt);
+    model_points<kFast>(P, area, misc, B, work, perm, sorted, yt);
     __syncthreads();
     if (tid < 3) yt[P.n_points + tid] = misc[M_CHK0 + tid];
     // relative-lightcurve normalisation of the model, mrqcof.c:53-58, 92-104

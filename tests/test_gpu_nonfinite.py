@@ -45,3 +45,16 @@ def test_rows(native, form, lmax, nrows):
         assert np.all(np.isposinf(y[:N][seen])) and np.all(y[:N][~seen] == 0), (log_cl, cls)
         assert np.all(np.isposinf(J[:N][seen, 0])) and np.all(J[:N][~seen, :C] == 0), (log_cl, cls)
     g.close()
+
+
+def test_fit_with_a_point_without_time(native):
+    """The point is dark in the model of every trial, as in the Jacobian's: the fit
+    takes steps, and its chi2 is the evaluation's at its parameters."""
+    d = _problem(3, 6, True, stop_condition=12.0)
+    g, _ = _open(native, "fp64", d)
+    for pole in (2, 7):
+        r, cg = g.fit(g.freq_start, pole, params=True)
+        assert r["niter"] == 12 and r["status"] == 0
+        assert np.isfinite(r["chisq"]) and r["chisq"] == g.mrqcof(cg)[2]
+        assert not np.array_equal(cg[:g.ncoef], g.array("cg_first"))  # some step was accepted
+    g.close()
