@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(32 * kCurvFacets) adj_curv(const DevProblem* _
 // facet by facet 45 % of the lanes were active and points in time order share
 // no facets to skip (20 000 points, 2048 facets: 174 us).  Where the FP32 sign
 // is wrong (a facet within 1e-6 of grazing) the pair's two facets are tested in
-// FP64.
-template <int K>
+// FP64.  A facet that is not seen counts with area 0; kMasked: with no terms, where
+// parameters or directions are so large that these may be infinite.
+template <int K, bool kMasked>
 __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
     __shared__ double sf[4 + K][2 * kPairChunk];  // nx, ny, nz, Area, z; [pair][side]
@@ -227,11 +228,14 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
         for (int c = 0; c < 3; c++) {
             e[c] = G.e[c];
             e0[c] = G.e0[c];
-            if (blockIdx.y == 0) {
+        }
+        if (!visible_geometry(e, e0))
+            for (int c = 0; c < 3; c++) e[c] = e0[c] = 0;
+        if (blockIdx.y == 0)
+            for (int c = 0; c < 3; c++) {
                 W.e6[(size_t)c * N + p] = e[c];
                 W.e6[(size_t)(3 + c) * N + p] = e0[c];
             }
-        }
     }
     const float e32[3] = {(float)e[0], (float)e[1], (float)e[2]};
     double acc[kFixed + K] = {};
@@ -262,6 +266,7 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
             }
             const double mu0 = fma(e0[2], nz, fma(e0[1], ny, e0[0] * nx));
             const bool vis = mu > kTinyD && mu0 > kTinyD;
+            if (kMasked && !vis) continue;
             const double ar = vis ? sf[3][i] : 0.0;
             const double r = rcp_newton(vis ? mu + mu0 : 1.0);
             const double am = ar * mu, am0 = ar * mu0, mm = am * mu0, cr = cls * r, crr = cr * r;
@@ -450,7 +455,8 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
 
 // q_f = sum_p ls_p s_pf over a block of points; thread per facet (neighbours
 // see nearly the same points), points staged in shared memory, two points at a
-// time without a branch.  Blocks of points small enough to fill the GPU: in
+// time without a branch (a facet that a point does not see adds zero times the
+// point's weight, nothing where a weight staged is not finite).  Blocks of points small enough to fill the GPU: in
 // blocks of 512, 760 points and 800 facets made 14 CTAs and 62 us.
 template <int K>
 __global__ void __launch_bounds__(kFcThreads) adj_facets(const DevProblem* __restrict__ Pp, AdjWork W) {
@@ -471,12 +477,15 @@ __global__ void __launch_bounds__(kFcThreads) adj_facets(const DevProblem* __res
     for (int b = p0; b < p1; b += kPtStage) {
         const int np = min(kPtStage, p1 - b), npu = (np + kU - 1) / kU * kU;
         __syncthreads();
+        bool fine = true;
         for (int i = threadIdx.x; i < npu * (6 + K); i += kFcThreads) {
             const int c = i / npu, j = i - c * npu;
             const double* src = c < 6 ? W.e6 + (size_t)c * N : W.ls + (size_t)(c - 6) * N;
-            sp[c][j] = j < np ? src[b + j] : 0.0;
+            const double v = j < np ? src[b + j] : 0.0;
+            fine = fine && isfinite(v);
+            sp[c][j] = v;
         }
-        __syncthreads();
+        fine = __syncthreads_and(fine);
         for (int i = 0; i < npu; i += kU) {
             double mu[kU], mu0[kU];
             bool vis[kU], some = false;
@@ -493,7 +502,8 @@ __global__ void __launch_bounds__(kFcThreads) adj_facets(const DevProblem* __res
                 const double r = rcp_newton(vis[u] ? mu[u] + mu0[u] : 1.0);
                 const double s = vis[u] ? mu[u] * mu0[u] * fma(cls, r, cl) : 0.0;
 #pragma unroll
-                for (int d = 0; d < K; d++) q[d] = fma(sp[6 + d][i + u], s, q[d]);
+                for (int d = 0; d < K; d++)
+                    if (fine || vis[u]) q[d] = fma(sp[6 + d][i + u], s, q[d]);
             }
         }
     }
@@ -608,7 +618,13 @@ cudaError_t launch(const DevProblem& P, const DevProblem* dP, double* work, cons
     W.chi2 = d_chi2;
     W.mode = mode;
     adj_curv<K><<<W.ncurv, 32 * kCurvFacets, 0, s>>>(dP, W, args);
-    adj_points<K><<<dim3(cdiv(P.n_points, kPtThreads), W.nfs), kPtThreads, 0, s>>>(dP, W);
+    bool masked = !ordinary_scattering(exp(args.a[P.C + 6]), args.a[P.C + 7]);
+    for (int k = 0; mode == kAdjProduct && k < P.C; k++) masked = masked || !(fabs(args.v[k]) < 1e200);
+    const dim3 pgrid(cdiv(P.n_points, kPtThreads), W.nfs);
+    if (masked)
+        adj_points<K, true><<<pgrid, kPtThreads, 0, s>>>(dP, W);
+    else
+        adj_points<K, false><<<pgrid, kPtThreads, 0, s>>>(dP, W);
     if (P.n_ablocks > 0) {
         adj_sums<K><<<P.n_ablocks, kRowThreads, 0, s>>>(dP, W);
         adj_rows<K, false><<<P.n_arows, kRowThreads, 0, s>>>(dP, W);

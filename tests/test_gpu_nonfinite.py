@@ -58,3 +58,37 @@ def test_fit_with_a_point_without_time(native):
         assert np.isfinite(r["chisq"]) and r["chisq"] == g.mrqcof(cg)[2]
         assert not np.array_equal(cg[:g.ncoef], g.array("cg_first"))  # some step was accepted
     g.close()
+
+
+@pytest.mark.parametrize("lmax,nrows", [(2, 4), (5, 7)])
+def test_matrix_free_calls(native, lmax, nrows):
+    """chi2, beta and products as the explicit evaluation has them: infinite where
+    the model is, finite in the shape columns where a point without a time is dark
+    (its rotation columns are not numbers in fused arithmetic)."""
+    d = _problem(lmax, nrows, True)
+    g, a = _open(native, "fast", d)
+    e, _ = _open(native, "fp64", d)
+    C, v = g.ncoef, np.ones(g.mfit)
+    alpha, beta, x2 = e.mrqcof(a)
+    x2_g, beta_g = g.chi2_grad(a)
+    assert abs(x2_g - x2) <= 1e-10 * x2
+    assert np.all(np.abs(beta_g - beta)[:C] <= 1e-10 * np.sqrt(np.diag(alpha) * x2)[:C])
+    for log_cl in (800.0, 705.0):
+        a[C + 6], a[C + 7] = log_cl, 1e308
+        x2_g, beta_g = g.chi2_grad(a)
+        assert np.isposinf(x2_g) and e.mrqcof(a)[2] == x2_g
+        assert not np.any(np.isfinite(beta_g[:C]))
+    g.close()
+    # an infinite weight: no finite chi2; an infinite brightness where no facet is
+    # seen: no facet's sum takes part in it
+    d = _problem(lmax, nrows, False)
+    d["weight"][DARK] = np.inf
+    g, a = _open(native, "fast", d)
+    assert not np.isfinite(g.chi2_grad(a)[0])
+    g.close()
+    d = _problem(lmax, nrows, False)
+    d["brightness"][DARK] = np.inf
+    g, a = _open(native, "fast", d)
+    x2_g, beta_g = g.chi2_grad(a)
+    assert np.isposinf(x2_g) and np.all(np.isfinite(beta_g[1:C]))
+    g.close()
