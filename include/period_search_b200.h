@@ -211,7 +211,8 @@ int ps_model(ps_ctx* ctx, const double* a, double* ymod, double* dyda);
 int ps_info(const ps_ctx* ctx, int* ints, double* dbls);
 /* Copy a host-setup array out (names as the oracle's pso_get_array:
  * "nor", "darea", "dsph", "cg_first", "ia", "tim", "ee", "ee0",
- * "brightness", "sig", "weight", "at", "af", "ifp").  Returns the element
+ * "brightness", "sig", "weight", "at", "af", "ifp"), or "pairs": the facets by
+ * antipodal pairs, as the matrix-free kernels take them.  Returns the element
  * count or -1. */
 int ps_get_array(const ps_ctx* ctx, const char* name, double* out);
 

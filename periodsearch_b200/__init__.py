@@ -309,7 +309,7 @@ class PeriodSearch:
         size = {"nor": 3 * self.numfac, "darea": self.numfac, "dsph": self.numfac * self.ncoef,
                 "cg_first": self.ncoef, "ia": self.ma, "tim": self.n_points, "ee": 3 * self.n_points,
                 "ee0": 3 * self.n_points, "brightness": self.n_points + 3, "sig": self.n_points + 3,
-                "weight": self.n_points + 3, "at": self.numfac, "af": self.numfac, "ifp": 3 * self.numfac}[name]
+                "weight": self.n_points + 3, "at": self.numfac, "af": self.numfac, "ifp": 3 * self.numfac, "pairs": self.numfac}[name]
         out = np.zeros(size)
         n = self._lib.ps_get_array(self._h, name.encode(), _dptr(out))
         if n < 0:
