@@ -1248,7 +1248,7 @@ int ps_get_array(const ps_ctx* c, const char* name, double* out) {
     if (!std::strcmp(name, "at")) return put(p.at);
     if (!std::strcmp(name, "af")) return put(p.af);
     if (!std::strcmp(name, "ifp")) return puti(p.ifp);
-    if (!std::strcmp(name, "pairs")) return puti(*p.pairs);
+    if (!std::strcmp(name, "pairs")) return p.pairs ? puti(*p.pairs) : -1;
     if (!std::strcmp(name, "brightness") || !std::strcmp(name, "sig") || !std::strcmp(name, "weight")) {
         const std::vector<double>& v = name[0] == 'b' ? p.brightness : (name[0] == 's' ? p.sig : p.weight);
         for (int i = 0; i < N; i++) out[i] = v[i];

@@ -156,8 +156,9 @@ int run(ps_batch* b, const int* n_from, const int* n_to, size_t* periods_out, cu
     if (fits > 0x7fffffff) return psb::set_error(PS_ERR_LIMIT, "too many fits in one batch scan");
     h[ctl_fit_off(n) + n] = (int)fits;
     h[ctl_per_off(n) + n] = (int)periods;
-    // longest fits first (cost ~ points x fits), so that the persistent
-    // kernel's last fits are short ones and the SMs finish together
+    // the asteroids with most work (points x fits) first, so that the persistent
+    // kernel's last fits tend to be short ones and the SMs finish together; with
+    // ranges of uneven length a long single fit may still come late
     std::vector<int> order(n);
     for (int a = 0; a < n; a++) order[a] = a;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {

@@ -710,7 +710,7 @@ __device__ __forceinline__ void model_facets(const double4* nrm, const double* e
 // on the way (four lanes of the last warp, facets in order).
 template <bool kFast>
 __device__ __forceinline__ void model_points(const DevProblem& P, const double* area, double* misc, const double* B,
-                                             double* work, int* perm, bool sorted, double* yt) {
+                                             const double* D, double* work, int* perm, bool sorted, double* yt) {
     constexpr int kU = 4;  // facets at a time
     const int tid = threadIdx.x, F = P.F, job = tid - (kThreads - 32);
     const double cl = misc[M_CL], cls = misc[M_CLS];
@@ -734,7 +734,7 @@ __device__ __forceinline__ void model_points(const DevProblem& P, const double* 
                 for (int c = 0; c < 3; c++) ej[j][c] = fj[j][c] = 0;
                 if (j < k && i < seg) {
                     PointGeom G;
-                    point_geometry(P, perm[i], B, B + 9, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
+                    point_geometry(P, perm[i], B, D, misc[M_OMG], misc[M_P1], misc[M_P2], misc[M_P3], G);
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
                         ej[j][c] = G.e[c];
@@ -813,7 +813,7 @@ __device__ void model_pass(const DevProblem& P, const double* a, double* g, doub
     eval_scalars(a, P.C, B, D, misc);
     curv_phase(P, a, g, area, false);
     __syncthreads();
-    model_points<kFast>(P, area, misc, B, work, perm, sorted, yt);
+    model_points<kFast>(P, area, misc, B, D, work, perm, sorted, yt);
     __syncthreads();
     if (tid < 3) yt[P.n_points + tid] = misc[M_CHK0 + tid];
     // relative-lightcurve normalisation of the model, mrqcof.c:53-58, 92-104
@@ -1339,7 +1339,7 @@ __global__ void __launch_bounds__(kThreads, NCB <= 64 ? 2 : 1) fit_kernel(const 
                 w = -1;
             } else if (Bt.n_ast > 1) {
                 // queue position -> asteroid; with an order, the queue runs over
-                // the asteroids in that order (largest first) and w becomes the
+                // the asteroids in that order (most work first) and w becomes the
                 // fit's index in the asteroid-ordered result array
                 const int* off = Bt.ast_order ? Bt.ast_ord_off : Bt.ast_fit_off;
                 int lo = 0, hi = Bt.n_ast - 1;  // last k with off[k] <= w
