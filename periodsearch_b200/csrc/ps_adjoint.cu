@@ -348,7 +348,7 @@ __device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W
 // each in turn: a gradient on one curve of 1000 / 5000 / 20 000 points and 800
 // facets 184 / 673 / 1313 us, 79 / 113 / 238 as a kernel of their own.  Where no
 // curve is longer, adj_rows forms the one block of its item itself and the
-// launch is saved: 60 calibrated points and 32 facets 58 against 62 us.
+// launch is saved: 40 calibrated points and 8 facets 58 against 62 us.
 template <int K>
 __global__ void __launch_bounds__(kRowThreads) adj_sums(const DevProblem* __restrict__ Pp, AdjWork W) {
     block_sums<K>(*Pp, W, reinterpret_cast<const int4*>(Pp->ablocks)[blockIdx.x]);

@@ -253,10 +253,11 @@ __device__ __forceinline__ void stage_chunk_async(const DevProblem& P, int f0, d
 // tiles with m8n8k4 FP64 MMAs (B = dsph rows from shared memory).  A step with
 // no visible (point, facet) pair skips its MMAs.  Out of line, for the
 // registers.  Bound by the latency of a step's chain and by instruction issue:
-// one reciprocal without a branch instead of the IEEE division's, and normals
-// read in pairs, took 2400 fits of 760 points, 800 facets and 49 coefficients
-// from 92.5 to 87.0 ms (two steps side by side: 90.7) and 140 fits of 20 000
-// points, 2048 facets and 81 coefficients, one CTA per SM, from 305 to 302.
+// one reciprocal without a branch (rcp_nearest) instead of the IEEE division's,
+// and normals read in pairs, took 2400 fits of 760 points, 800 facets and 49
+// coefficients from 92.5 to 88.0 ms (two steps side by side: 4 % slower) and 140
+// fits of 20 000 points, 2048 facets and 81 coefficients, one CTA per SM, from 305
+// to 303.
 // Facet chunks are staged with asynchronous copies, one chunk ahead.  Sums
 // split by facet (lane q takes facets q mod 4) are combined at the end: the form
 // differs from the reference order by rounding only.
@@ -872,12 +873,13 @@ __device__ __noinline__ void evaluate_model(const DevProblem* __restrict__ Pp, i
 // points, 800 facets and 49 coefficients: 314 ms with one facet at a time, three
 // or four IEEE divisions each, inlined; 277 with two facets and one reciprocal;
 // 261 out of line; 253 with the halves balanced (ref_halves; one facet: 286,
-// four: 276, which need more than 128 registers).  With few coefficients
-// (kFlat) registers are left to run the sums' products side by side too, and
-// the pass is a chain of latencies: one fit of 118 points and 16 coefficients
-// 6.3 -> 5.8 ms, the pre-pass and 400 fits of 500 points 104 -> 97 ms; 290 fits
-// of 500 points and 25 coefficients 34.3 -> 32.3, of 700 and 36 60 -> 58; at 49
-// coefficients 249 -> 256.
+// four: 276, which need more than 128 registers); 247 with the present
+// reciprocal and without what only evaluations need (kAll).  With few
+// coefficients (kFlat) registers are left to run the sums' products side by side
+// too, and the pass is a chain of latencies: one fit of 118 points and 16
+// coefficients is 8 % faster, the pre-pass and 400 fits of 500 points 7 %, 290
+// fits of 500 points and 25 coefficients 6 %, of 700 and 36 3 %; at 49
+// coefficients 3 % slower.
 // `p`: the thread's point, -1 for none.  first: also the facet sums.  want_cl:
 // also the column of the Lambert coefficient.  kAll: also that of the
 // Lommel-Seeliger coefficient, which no fit varies, and any value of it (fits
