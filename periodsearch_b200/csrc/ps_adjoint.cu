@@ -358,7 +358,9 @@ __global__ void __launch_bounds__(kRowThreads) adj_sums(const DevProblem* __rest
 // calibrated points, or (the last) the three convexity rows.  Per relative
 // lightcurve ave = sum y and S = sum J v without v_1 (mrqcof.c:53-58, 92-104);
 // per row the normalised model and J v, the residual, u = W (y_obs - y') or
-// W J' v, and the item's share of chi2; the adjoint weights l.  kOwnSums: the
+// W J' v, and the item's share of chi2; the adjoint weights l.  (y S) / ave in
+// mrqcof's order: where it overflows, as at a Lambert coefficient of 1e200, J' is
+// infinite there and a fit freezes.  kOwnSums: the
 // item is one block, whose sums are formed here (see adj_sums).
 template <int K, bool kOwnSums>
 __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __restrict__ Pp, AdjWork W) {
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         ave = block_sum(sy, red);
         coefn = (double)item.w / ave;
 #pragma unroll
-        for (int d = 0; d < K; d++) sjv[d] = block_sum(sj[d], red) / ave;
+        for (int d = 0; d < K; d++) sjv[d] = block_sum(sj[d], red);
     }
     for (int p = item.x + tid; p < item.y; p += kRowThreads) {
         const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0, rs = rel ? P.sig[p] / sig0 : 1.0;
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
 #pragma unroll
         for (int d = 0; d < K; d++) {
             const double jv = W.jv[(size_t)d * N + p];
-            const double u = W.mode == kAdjGradient ? w * dy : w * (rel ? coef * (jv - y * sjv[d]) : jv);
+            const double u = W.mode == kAdjGradient ? w * dy : w * (rel ? coef * (jv - y * sjv[d] / ave) : jv);
             W.lam[(size_t)d * N + p] = u;
             kap[d] = fma(rs * y, u, kap[d]);
         }

@@ -92,3 +92,23 @@ def test_matrix_free_calls(native, lmax, nrows):
     x2_g, beta_g = g.chi2_grad(a)
     assert np.isposinf(x2_g) and np.all(np.isfinite(beta_g[1:C]))
     g.close()
+
+
+@pytest.mark.parametrize("seed,lmax,nrows,poles", [(3, 3, 6, (6, 7)), (21, 1, 4, (5, 10))])
+def test_fits_that_run_into_overflow(native, seed, lmax, nrows, poles):
+    """Relative lightcurves alone do not determine the Lambert coefficient: these
+    fits run to exp(355) and more, where y sum(dy) overflows in the normalisation,
+    and freeze with a matrix of NaNs (status 1).  The Jacobian-free fit does too."""
+    d = _desc(2000 + seed, [(1, 40), (1, 30)], lmax, nrows, False)
+    d.update(stop_condition=6.0, per_start=7.9, per_end=8.1, weight=np.ones(70))
+    g, _ = _open(native, "fp64", d)
+    f, _ = _open(native, "fast", d)
+    for pole in poles:
+        r, cg = g.fit(g.freq_start, pole, params=True)
+        assert r["status"] == 1 and cg[g.ncoef + 6] > 355
+        j = f.fit_jfree(g.freq_start, pole)
+        assert j["status"] == 1 and j["niter"] == r["niter"]
+        assert abs(j["chisq"] - r["chisq"]) <= 1e-9 * r["chisq"]
+        assert not np.any(np.isfinite(f.gn_product(cg, np.ones(f.mfit))))
+    g.close()
+    f.close()
