@@ -25,10 +25,10 @@
 // Six kernels, or seven, each spread over the GPU by how many CTAs its sizes give:
 // adj_curv (warp per facet: scalars, areas, z, facet sums), adj_points (point
 // blocks x facet slices), adj_sums (CTA per block of points of one curve: the
-// slices' sums, model, columns of J; part of adj_rows where every curve is one
-// block), adj_rows (CTA per relative lightcurve or
-// block of calibrated points: residual, adjoint weights), adj_facets (facet blocks x point blocks), adj_cols (blocks of facets: the
-// F x C contraction), adj_out (CTA per free parameter).
+// slices' sums, model, columns of J; part of adj_rows where no relative curve is
+// long), adj_rows (CTA per relative lightcurve or block of calibrated points:
+// residual, adjoint weights), adj_facets (facet blocks x point blocks), adj_cols
+// (blocks of facets: the F x C contraction), adj_out (CTA per free parameter).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -293,17 +293,18 @@ __global__ void __launch_bounds__(kPtThreads) adj_points(const DevProblem* __res
 // A block of at most kAdjRowBlock points of one lightcurve, by kRowThreads
 // threads: the slices' sums in slice order, kRowThreads / kAdjRowBlock threads
 // per point, then a thread per point the model, the non-shape columns of J and
-// J v.
+// J v; the thread's y and J v are added to sy and sj.
 template <int K>
-__device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W, const int4& item) {
+__device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W, int first, int last, bool rel,
+                                           double& sy, double* sj) {
     __shared__ double sums[kFixed + K][kAdjRowBlock];
     const int tid = threadIdx.x, N = P.n_points;
     const double* x = W.misc;
     const double cl = x[X_CL];
-    const int np = item.y - item.x, i0 = tid % kAdjRowBlock;
+    const int np = last - first, i0 = tid % kAdjRowBlock;
     if (i0 < np)
         for (int j = tid / kAdjRowBlock; j < kFixed + K; j += kRowThreads / kAdjRowBlock) {
-            const double* src = W.pp + (size_t)j * W.nfs * N + item.x + i0;
+            const double* src = W.pp + (size_t)j * W.nfs * N + first + i0;
             double v = 0;
 #pragma unroll 8
             for (int k = 0; k < W.nfs; k++) v += src[(size_t)k * N];
@@ -311,7 +312,7 @@ __device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W
         }
     __syncthreads();
     if (tid >= np) return;
-    const int p = item.x + tid;
+    const int p = first + tid;
     PointGeom G;
     point_geometry(P, p, x + X_B, x + X_D, x[X_OMG], x[X_P1], x[X_P2], x[X_P3], G);
     double acc[kFixed + K];
@@ -329,29 +330,35 @@ __device__ __forceinline__ void block_sums(const DevProblem& P, const AdjWork& W
     jn[5] = br * G.dphp[2];
     jn[6] = sc * acc[1] * cl;
     jn[7] = sc * acc[2];
-    jn[8] = item.z ? 0.0 : yy;  // first shape coefficient
+    jn[8] = rel ? 0.0 : yy;  // first shape coefficient
     for (int j = 0; j < 9; j++) W.jns[(size_t)j * N + p] = jn[j];
     W.y[p] = yy;
     W.scale[p] = sc;
+    sy += yy;
 #pragma unroll
     for (int d = 0; d < K; d++) {
         const double* v = W.dir + 9 * d;
         double s = jn[8] * v[0];
         for (int j = 0; j < 8; j++) s = fma(jn[j], v[1 + j], s);
-        W.jv[(size_t)d * N + p] = fma(sc, acc[kFixed + d], s);
+        s = fma(sc, acc[kFixed + d], s);
+        W.jv[(size_t)d * N + p] = s;
+        sj[d] += s;
     }
 }
 
-// A block of points per CTA, where some relative lightcurve is longer than a
-// block: its own kernel, whose blocks spread over the GPU however long a
-// lightcurve is.  Inside adj_rows, a CTA per relative lightcurve, they took 3 us
-// each in turn: a gradient on one curve of 1000 / 5000 / 20 000 points and 800
-// facets 184 / 673 / 1313 us, 79 / 113 / 238 as a kernel of their own.  Where no
-// curve is longer, adj_rows forms the one block of its item itself and the
-// launch is saved: 40 calibrated points and 8 facets 58 against 62 us.
+// A block of points per CTA, where some relative lightcurve is longer than
+// kAdjOwnBlocks of them: its own kernel, whose blocks spread over the GPU however
+// long a lightcurve is.  Inside adj_rows, a CTA per relative lightcurve, they took
+// 3 us each in turn: a gradient on one curve of 1000 / 5000 / 20 000 points and
+// 800 facets 184 / 673 / 1313 us, 79 / 113 / 238 as a kernel of their own.  Where
+// no curve is longer, adj_rows forms its item's blocks itself and the launch is
+// saved, which costs as much as two blocks in turn: 40 calibrated points and 8
+// facets 58 against 62 us, two nights of 80 points among 760 73 against 76.
 template <int K>
 __global__ void __launch_bounds__(kRowThreads) adj_sums(const DevProblem* __restrict__ Pp, AdjWork W) {
-    block_sums<K>(*Pp, W, reinterpret_cast<const int4*>(Pp->ablocks)[blockIdx.x]);
+    const int4 item = reinterpret_cast<const int4*>(Pp->ablocks)[blockIdx.x];  // first point, last + 1, relative
+    double sy = 0, sj[K] = {};  // adj_rows forms the curve's
+    block_sums<K>(*Pp, W, item.x, item.y, item.z != 0, sy, sj);
 }
 
 // One item of the row list per CTA: a relative lightcurve, a block of
@@ -360,8 +367,8 @@ __global__ void __launch_bounds__(kRowThreads) adj_sums(const DevProblem* __rest
 // per row the normalised model and J v, the residual, u = W (y_obs - y') or
 // W J' v, and the item's share of chi2; the adjoint weights l.  (y S) / ave in
 // mrqcof's order: where it overflows, as at a Lambert coefficient of 1e200, J' is
-// infinite there and a fit freezes.  kOwnSums: the
-// item is one block, whose sums are formed here (see adj_sums).
+// infinite there and a fit freezes.  kOwnSums: the item's blocks are formed here
+// (see adj_sums).
 template <int K, bool kOwnSums>
 __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __restrict__ Pp, AdjWork W) {
     const DevProblem& P = *Pp;
@@ -397,15 +404,16 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         if (tid == 0) W.x2part[blockIdx.x] = x2;
         return;
     }
-    if constexpr (kOwnSums) {
-        block_sums<K>(P, W, item);
-        __syncthreads();
-    }
     const bool rel = item.z != 0;
     double sy = 0, sj[K];
 #pragma unroll
     for (int d = 0; d < K; d++) sj[d] = 0;
-    if (rel) {
+    if constexpr (kOwnSums) {
+        for (int p = item.x; p < item.y; p += kAdjRowBlock) {
+            block_sums<K>(P, W, p, min(p + kAdjRowBlock, item.y), rel, sy, sj);
+            __syncthreads();
+        }
+    } else if (rel) {
 #pragma unroll 2
         for (int p = item.x + tid; p < item.y; p += kRowThreads) {
             sy += W.y[p];
@@ -417,6 +425,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
     // for the per-curve mean
     double ave = 0, sjv[K], kap[K], coefn = 0;
     const double sig0 = rel ? P.sig[item.x] : 1.0;
+    auto ratio = [&](double sig) { return sig == sig0 ? 1.0 : sig / sig0; };
 #pragma unroll
     for (int d = 0; d < K; d++) sjv[d] = kap[d] = 0;
     if (rel) {
@@ -426,7 +435,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         for (int d = 0; d < K; d++) sjv[d] = block_sum(sj[d], red);
     }
     for (int p = item.x + tid; p < item.y; p += kRowThreads) {
-        const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0, rs = rel ? P.sig[p] / sig0 : 1.0;
+        const double y = W.y[p], coef = rel ? P.sig[p] * coefn : 1.0, rs = rel ? ratio(P.sig[p]) : 1.0;
         const double w = P.sig2i[p] * P.wght[p], dy = P.yobs[p] - coef * y;
         x2 = fma(dy * w, dy, x2);
 #pragma unroll
@@ -442,7 +451,7 @@ __global__ void __launch_bounds__(kRowThreads) adj_rows(const DevProblem* __rest
         for (int d = 0; d < K; d++) kap[d] = block_sum(kap[d], red) / ave;
     }
     for (int p = item.x + tid; p < item.y; p += kRowThreads) {
-        const double sc = W.scale[p], coef0 = sig0 * coefn, rs = rel ? P.sig[p] / sig0 : 1.0;
+        const double sc = W.scale[p], coef0 = sig0 * coefn, rs = rel ? ratio(P.sig[p]) : 1.0;
 #pragma unroll
         for (int d = 0; d < K; d++) {
             double l = W.lam[(size_t)d * N + p];

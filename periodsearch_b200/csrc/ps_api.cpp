@@ -306,8 +306,9 @@ int upload_static(ps_ctx* c) {
             ints.insert(ints.end(), {r, std::min(r + block, lc_start[i + 1]), p.lc_rel[i], p.lc_points[i]});
     };
     const size_t block_at = ints.size();
-    bool longer = false;  // than a block: some relative lightcurve
-    for (int i = 0; i < L; i++) longer = longer || (p.lc_rel[i] && p.lc_points[i] > psb::kAdjRowBlock);
+    bool longer = false;  // than one CTA should take: some relative lightcurve
+    for (int i = 0; i < L; i++)
+        longer = longer || (p.lc_rel[i] && p.lc_points[i] > psb::kAdjOwnBlocks * psb::kAdjRowBlock);
     for (int i = 0; longer && i < L; i++) cut(i, psb::kAdjRowBlock);
     const size_t row_at = ints.size();
     for (int i = 0; i < L; i++) cut(i, p.lc_rel[i] ? p.lc_points[i] : psb::kAdjRowBlock);

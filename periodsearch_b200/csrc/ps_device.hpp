@@ -8,6 +8,7 @@
 namespace psb {
 
 constexpr int kAdjRowBlock = 64;  // points of one block of the matrix-free lists
+constexpr int kAdjOwnBlocks = 2;  // blocks of a relative lightcurve that one CTA may take in turn
 
 // Per-asteroid tables, all device pointers, 0-based.
 //  rows: n_points data rows (lightcurve order) followed by 3 convexity rows.
@@ -32,8 +33,9 @@ struct DevProblem {
     const double* pole0;     // [10][2]: initial beta' and lambda [rad]
     // matrix-free form: facets by antipodal pairs [F/2][2]; blocks of the points
     // of each lightcurve {first, last + 1, relative, points of the lightcurve}, none
-    // if no relative lightcurve is longer than one; row items, likewise: each relative lightcurve, blocks of the calibrated
-    // ones, the convexity rows
+    // if no relative lightcurve is longer than kAdjOwnBlocks of them; row items,
+    // likewise: each relative lightcurve, blocks of the calibrated ones, the
+    // convexity rows
     const int* apair;
     const int* ablocks;
     const int* arows;

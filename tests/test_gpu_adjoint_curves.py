@@ -63,7 +63,7 @@ def test_sigma_varying_within_a_curve(native, curves, lmax, nrows):
     _check(native, _desc(3, curves, lmax, nrows, True), 4)
 
 
-@pytest.mark.parametrize("curves,lmax,nrows", [([(1, 64)], 2, 3), ([(0, 64), (1, 129)], 3, 4),
+@pytest.mark.parametrize("curves,lmax,nrows", [([(1, 64)], 2, 3), ([(1, 65), (0, 70), (1, 128)], 3, 4), ([(0, 64), (1, 129)], 3, 4),
                                                ([(1, 255), (1, 256), (0, 257), (1, 700)], 4, 5), ([(1, 5000)], 6, 10)])
 def test_curves_longer_than_a_block(native, curves, lmax, nrows):
     _check(native, _desc(5, curves, lmax, nrows, False), 6)
